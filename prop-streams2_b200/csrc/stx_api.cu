@@ -135,6 +135,58 @@ int upload(stx_ctx *c, const T *host, size_t n, const T **out) {
   return STX_OK;
 }
 
+// The packed reaction records of chem_source_rec.  A mechanism has them when every
+// reaction is plain, three-body, Lindemann or Troe, has integer stoichiometry of
+// at most REC_SLOTS molecules a side and at most REC_NET net species; otherwise
+// t.rec stays null and the sparse lists serve it.
+int upload_records(stx_ctx *c, const stx_tables *tab, DevTab &t) {
+  const int ns = t.ns, nr = t.nr;
+  t.rec = t.rec_eff = nullptr;
+  t.rec_es = (ns + 1) & ~1;
+  if (ns > 200) return STX_OK;
+  std::vector<double> rec((size_t)nr * REC_N, 0.0), eff((size_t)nr * t.rec_es, 0.0);
+  for (int r = 0; r < nr; r++) {
+    double *R = &rec[(size_t)r * REC_N];
+    const int ty = tab->reac_ty[r];
+    if (ty < 0 || ty > 3) return STX_OK;
+    int cls = ty == 0 ? REC_PLAIN : ty == 1 ? REC_TB : ty == 2 ? REC_LIND : REC_TROE;
+    R[0] = tab->arr_a[r]; R[1] = tab->arr_b[r]; R[2] = -tab->arr_ea[r];
+    R[4] = tab->arr_a[nr + r]; R[5] = tab->arr_b[nr + r]; R[6] = -tab->arr_ea[nr + r];
+    if (ty == 3) {
+      // Fcent = (1 - F1) exp(-T/F2) + F1 exp(-T/F3) [+ exp(-F4/T)] is F1 in double
+      // precision for 1 <= T <= 1e6 where F2 is tiny and F3 and F4 are huge
+      const double F1 = tab->falloff[r], F2 = tab->falloff[nr + r], F3 = tab->falloff[2 * nr + r],
+                   F4 = tab->falloff[3 * nr + r];
+      if (F1 > 0.0 && F2 > 0.0 && F2 <= 1e-20 && F3 >= 1e25 && (F4 == -3.14 || F4 >= 1e10)) {
+        cls = REC_TROE_C;
+        R[3] = F1;
+      }
+    }
+    unsigned char ix[16];
+    for (int q = 0; q < 16; q++) ix[q] = (unsigned char)ns;
+    int nR = 0, nP = 0, nU = 0;
+    for (int k = 0; k < ns; k++) {
+      const double rr = tab->r_coeffs[(size_t)k * nr + r], pp = tab->p_coeffs[(size_t)k * nr + r];
+      if (!(rr >= 0.0 && rr <= REC_SLOTS && pp >= 0.0 && pp <= REC_SLOTS) || rr != (int)rr || pp != (int)pp)
+        return STX_OK;
+      if (nR + (int)rr > REC_SLOTS || nP + (int)pp > REC_SLOTS) return STX_OK;
+      for (int q = 0; q < (int)rr; q++) ix[nR++] = (unsigned char)k;
+      for (int q = 0; q < (int)pp; q++) ix[REC_SLOTS + nP++] = (unsigned char)k;
+      if (rr != pp) {
+        if (nU == REC_NET) return STX_OK;
+        ix[2 * REC_SLOTS + nU] = (unsigned char)k;
+        R[8 + nU++] = (pp - rr) * tab->mw[k];
+      }
+      eff[(size_t)r * t.rec_es + k] = tab->tb_eff[(size_t)k * nr + r];
+    }
+    const int flag[2] = {cls | (tab->is_rev[r] == 1) << 8 | nU << 16, 0};   // low word first
+    std::memcpy(R + 7, flag, sizeof flag);
+    std::memcpy(R + 14, ix, sizeof ix);
+  }
+  int rc = upload(c, rec.data(), rec.size(), &t.rec);
+  return rc ? rc : upload(c, eff.data(), eff.size(), &t.rec_eff);
+}
+
 bool ns_supported(int ns) {
 #define X(N) if (ns == N) return true;
   STX_FOR_NS(X)
@@ -273,6 +325,26 @@ static int ctx_create_impl(const stx_params *par, const stx_tables *tab, const s
   if ((rc = upload(c, tab->trange, (size_t)ns * (t.nset + 1), &t.trange))) return fail(rc);
   if ((rc = upload(c, tab->cp_coeff, (size_t)t.ncp * ns * t.nset, &t.cp))) return fail(rc);
   if ((rc = upload(c, tab->cv_coeff, (size_t)t.ncp * ns * t.nset, &t.cv))) return fail(rc);
+  // two ranges, powers 0..4: the fast T(e) and cp paths (mix_poly2)
+  t.poly2 = t.icl == 0 && t.icr == 4 && t.nset == 2 && ns <= 64;
+  t.umid = tab->trange[ns];
+  for (int k = 1; k < ns; k++)
+    if (tab->trange[ns + k] != t.umid) t.umid = -1.0;
+  if (!(t.umid >= 0.0)) t.umid = -1.0;
+  t.cp6 = t.cv6 = t.cpi6 = nullptr;
+  if (t.poly2) {
+    std::vector<double> p6((size_t)6 * ns * 2), v6((size_t)6 * ns * 2);
+    for (size_t q = 0; q < (size_t)ns * 2; q++)
+      for (int l = 0; l < 6; l++) {
+        p6[q * 6 + l] = tab->cp_coeff[q * t.ncp + l];
+        v6[q * 6 + l] = tab->cv_coeff[q * t.ncp + l];
+      }
+    if ((rc = upload(c, p6.data(), p6.size(), &t.cp6))) return fail(rc);
+    if ((rc = upload(c, v6.data(), v6.size(), &t.cv6))) return fail(rc);
+    for (size_t q = 0; q < (size_t)ns * 2; q++)
+      for (int l = 0; l < 5; l++) p6[q * 6 + l] = p6[q * 6 + l] / (l + 1.0);
+    if ((rc = upload(c, p6.data(), p6.size(), &t.cpi6))) return fail(rc);
+  }
   {
     // integrated tables: coef_l / (l + 1) for the terms l >= 0 of h(T) and e(T)
     // (the quotient the reference forms per evaluation, get_species_h_from_temperature_dev)
@@ -367,6 +439,7 @@ static int ctx_create_impl(const stx_params *par, const stx_tables *tab, const s
       if ((rc = upload(c, kr.data(), kr.size(), &t.sk_r))) return fail(rc);
       if ((rc = upload(c, kc.data(), kc.size(), &t.sk_c))) return fail(rc);
     }
+    if ((rc = upload_records(c, tab, t))) return fail(rc);
     std::vector<double> kr(ntab1 * nr);
     for (size_t it = 0; it < ntab1; it++)
       for (int r = 0; r < nr; r++) kr[it * nr + r] = tab->kc_tab[(size_t)r * ntab1 + it];

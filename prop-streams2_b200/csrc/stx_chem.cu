@@ -18,6 +18,12 @@
 #define STX_ROK4_MINB 4
 #endif
 
+// Grids of at most this many cells take a warp per cell (k_rok4_w): the bits are
+// the same, and a thread per cell leaves most of the chip idle there.
+#ifndef STX_ROK4_WARP_CELLS
+#define STX_ROK4_WARP_CELLS 8192
+#endif
+
 // cg: a device-resident copy of c.  The right-hand side is one out-of-line
 // function that takes the context by reference; given the kernel parameter c,
 // every thread would keep its own local copy of the whole context (~0.9 KB),
@@ -124,14 +130,14 @@ __device__ void ros_rhs(const DevCtx &c, double *wc, double *Y, double &T, doubl
 #pragma unroll
   for (int m = 0; m < NS + 4; m++) rhs[m] = 0.0;
   constexpr int CB = chem_block(NS);
-  __shared__ double s_conc[NS * CB], s_rhs[NS * CB];
+  __shared__ double s_conc[(NS + 1) * CB], s_rhs[(NS + 1) * CB];
   double *cs = s_conc + threadIdx.x, *rs = s_rhs + threadIdx.x;
 #pragma unroll
   for (int k = 0; k < NS; k++) {
     cs[k * CB] = conc[k];
     rs[k * CB] = 0.0;
   }
-  chem_source_sp<NS, CB>(t, T, cs, rs);
+  chem_source_rows<NS, CB, false>(t, T, cs, rs);
 #pragma unroll
   for (int k = 0; k < NS; k++) rhs[k] = rs[k * CB];
 }
@@ -370,6 +376,10 @@ int chem_ctas_limit(int ns) {
 template <int NS>
 static int rok4_t(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa, const double *fl_sav,
                   double dttry, double t0, double t1, int simpler, unsigned int *counter) {
+  if (c.g.npi <= STX_ROK4_WARP_CELLS) {
+    int rc = launch_rok4_warp(c, cg, s, w, wa, fl_sav, dttry, t0, t1, simpler);
+    if (rc != STX_E_UNSUPPORTED) return rc;
+  }
   long long need = (c.g.npi + chem_block(NS) - 1) / chem_block(NS);
   if (c.p.chem_ctas_per_sm < 0) {            // the plain launch: a thread per cell, no work stealing
     k_rok4<NS><<<(unsigned)need, chem_block(NS), 0, s>>>(c, cg, w, wa, fl_sav, dttry, t0, t1, simpler, nullptr);

@@ -26,6 +26,16 @@
 __host__ __device__ constexpr int chem_block(int ns) { return ns > 20 ? 32 : 128; }
 __host__ __device__ constexpr int xsweep_block(int ns) { return ns > 20 ? 64 : 128; }
 
+// One packed reaction (chem_source_rec), 128 bytes, read with 16-byte loads:
+//   0 A, 1 b, 2 -E of k (k0 of a fall-off form); 3 Fcent where it is constant
+//   4 A, 5 b, 6 -E of k_inf; 7 class | reversible << 8 | number of net species << 16 (an int)
+//   8..13 (nu'' - nu')_k W_k of the net species
+//   14 bytes: reactants 0..2, products 3..5, net species 6..11 (species count: none)
+#define REC_N 16
+#define REC_SLOTS 3        // reactant (or product) molecules of a reaction
+#define REC_NET 6          // net species of a reaction
+enum { REC_PLAIN = 0, REC_TB = 1, REC_LIND = 2, REC_TROE_C = 3, REC_TROE = 4 };
+
 struct DevTab {
   int ns, nr, icl, icr, nset, ntab, ncp;
   double tmin, dtab, Ru;
@@ -53,6 +63,16 @@ struct DevTab {
   const int *sk_r;
   const double *sk_c;
   const double *wk_a, *wk_b;      // Wilke pair factors [l][m]
+  // poly2: the property polynomials are the two-range form with powers 0..4
+  // (the 7-coefficient NASA form), which the fast T(e) and cp paths take;
+  // umid: its middle temperature, where every species has the same (else < 0)
+  int poly2;
+  double umid;
+  const double *cp6, *cv6, *cpi6; // (6, ns, nset): the powers 0..4 and the constant of cp, cv and cpi
+  // packed reaction records [lr][REC_N] and third-body rows [lr][rec_es] of
+  // chem_source_rec; null where a reaction does not fit the record
+  const double *rec, *rec_eff;
+  int rec_es;
   int n_eoi;
   const double *aw_eoi, *coeff_eoi, *beta0;
   const int *nainsp;
@@ -154,9 +174,108 @@ __device__ __forceinline__ int locate_range(const DevTab &t, double T, int lsp) 
   return jl;
 }
 
+// ---- the two-range form with powers 0..4 (DevTab::poly2).  With the mass
+// fractions fixed, the mixture is one polynomial of T: its coefficients
+// sum_k a_lk Y_k, summed over the species in the order of the general path, are
+// formed once and serve every Newton iteration until T crosses a species' middle
+// temperature, where the general path gathers all of them (6 NS loads with run-time
+// addresses) in each iteration.  Each species' row is three 16-byte loads; where all species share the
+// middle temperature the two possible rows lie at fixed offsets.  Same bits as
+// the general path.
+__device__ __forceinline__ bool range_next(bool hi, double T, double mid) { return hi ? !(T < mid) : T > mid; }
+
+template <int NS>
+__device__ __forceinline__ void mix_poly2(const DevTab &t, const double *coef, unsigned long long hi, const double *Y,
+                                          double *a) {
+#pragma unroll
+  for (int l = 0; l < 6; l++) a[l] = 0.0;
+  if (t.umid >= 0.0) {
+    const double2 *b = (const double2 *)(coef + (hi ? NS * 6 : 0));
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+      const double2 u = __ldg(b + 3 * k), v = __ldg(b + 3 * k + 1), x = __ldg(b + 3 * k + 2);
+      a[0] = a[0] + u.x * Y[k]; a[1] = a[1] + u.y * Y[k]; a[2] = a[2] + v.x * Y[k];
+      a[3] = a[3] + v.y * Y[k]; a[4] = a[4] + x.x * Y[k]; a[5] = a[5] + x.y * Y[k];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+      const double2 *b = (const double2 *)(coef + k * 6 + ((hi >> k) & 1ull ? NS * 6 : 0));
+      const double2 u = __ldg(b), v = __ldg(b + 1), x = __ldg(b + 2);
+      a[0] = a[0] + u.x * Y[k]; a[1] = a[1] + u.y * Y[k]; a[2] = a[2] + v.x * Y[k];
+      a[3] = a[3] + v.y * Y[k]; a[4] = a[4] + x.x * Y[k]; a[5] = a[5] + x.y * Y[k];
+    }
+  }
+}
+
+// the species whose upper range holds T (bit k; any bit where all share umid)
+template <int NS>
+__device__ __forceinline__ unsigned long long mid_mask(const DevTab &t, double T) {
+  if (t.umid >= 0.0) return T >= t.umid ? 1ull : 0ull;
+  unsigned long long m = 0;
+#pragma unroll
+  for (int k = 0; k < NS; k++) m |= T >= ldg(t.trange + NS + k) ? 1ull << k : 0ull;
+  return m;
+}
+
+template <int NS>
+__device__ __forceinline__ double mix_cp2(const DevTab &t, double tt, const double *Y) {
+  double a[6];
+  mix_poly2<NS>(t, t.cp6, mid_mask<NS>(t, tt), Y, a);
+  double cploc = 0.0, pw = 1.0;
+#pragma unroll
+  for (int l = 0; l <= 4; l++) {
+    cploc = cploc + a[l] * pw;
+    pw = pw * tt;
+  }
+  return cploc;
+}
+
+template <int NS>
+__device__ __forceinline__ double temp_from_poly2(const DevTab &t, const double *coef, const DevPar &p, double ee,
+                                                  double T_start, const double *Y) {
+  unsigned long long hi = mid_mask<NS>(t, T_start);
+  double a[6];
+  double T_old = T_start, tt = T_start;
+  bool conv = false;
+#pragma unroll 1
+  for (int iter = 1; iter <= 10; iter++) {
+    bool fresh = iter == 1;
+    if (iter > 1) {
+      unsigned long long h2 = 0;
+      if (t.umid >= 0.0) {
+        h2 = range_next(hi != 0, T_old, t.umid) ? 1ull : 0ull;
+      } else {
+#pragma unroll
+        for (int k = 0; k < NS; k++)
+          h2 |= range_next((hi >> k) & 1ull, T_old, ldg(t.trange + NS + k)) ? 1ull << k : 0ull;
+      }
+      fresh = h2 != hi;
+      hi = h2;
+    }
+    if (fresh) mix_poly2<NS>(t, coef, hi, Y, a);
+    const double ebar = ee - a[5];
+    double den = 0.0, num = 0.0, pw = 1.0;
+#pragma unroll
+    for (int l = 0; l <= 4; l++) {
+      const double tn = T_old * pw;
+      const double tnum = l == 0 ? tn : (l == 1 ? tn * 0.5 : (l == 3 ? tn * 0.25 : tn / (l + 1.0)));
+      num = num + a[l] * tnum;
+      den = den + a[l] * pw;
+      pw = pw * T_old;
+    }
+    tt = T_old + (ebar - num) / den;
+    if (fabs(tt - T_old) < p.tol) { conv = true; break; }
+    T_old = tt;
+  }
+  if (!conv) set_status(p, STX_ST_NEWTON_CAP);
+  return tt;
+}
+
 // get_cp_dev (kernels_gpu.F90:6384-6432)
 template <int NS>
 __device__ double mix_cp(const DevTab &t, double tt, const double *Y) {
+  if (t.poly2) return mix_cp2<NS>(t, tt, Y);
   int nrange[NS];
 #pragma unroll
   for (int k = 0; k < NS; k++) nrange[k] = 1;
@@ -197,6 +316,7 @@ __device__ __forceinline__ double temp_from_e(const DevTab &t, const DevPar &p, 
 template <int NS>
 __device__ double temp_from_poly(const DevTab &t, const double *coef, const DevPar &p, double ee, double T_start,
                                  const double *Y) {
+  if (t.poly2) return temp_from_poly2<NS>(t, coef == t.cp ? t.cp6 : t.cv6, p, ee, T_start, Y);
   int nrange[NS];
 #pragma unroll
   for (int k = 0; k < NS; k++) nrange[k] = 1;

@@ -57,6 +57,9 @@ int chem_ctas_limit(int ns);
 // cg: the device-resident copy of c (stx_ctx::dctx_d)
 int launch_rok4(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa, const double *fl_sav,
                 double dttry, double t0, double t1, int simpler, unsigned int *counter);
+// the same with a warp per cell, for small grids (STX_E_UNSUPPORTED: not for this mechanism)
+int launch_rok4_warp(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa,
+                     const double *fl_sav, double dttry, double t0, double t1, int simpler);
 int launch_rosenbrock(const DevCtx &c, cudaStream_t s, double *w, double *wa, double dttry, double t0, double t1,
                       unsigned int *counter);
 int launch_chem_explicit(const DevCtx &c, cudaStream_t s, double *w, double *wa, double *fl);

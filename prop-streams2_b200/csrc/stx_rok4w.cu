@@ -1,23 +1,22 @@
 // stx_rok4w.cu -- the ROK4 integration (kernels_gpu.F90:10360-11205) with one
-// warp per state vector, for the batched 0-D reactors.
+// warp per state vector, for the batched 0-D reactors and for small grids.
 //
 // The thread-per-cell kernels suit large grids: 32 cells per warp amortise the
-// Krylov algebra.  A batch of reactors is different: the reactors that ignite
-// late take tens of thousands of steps, and the launch lasts as long as the
-// slowest one, integrated serially by a single thread.  Here a warp integrates
-// one reactor:
+// Krylov algebra.  A batch of reactors or a grid of a few thousand cells is
+// different: a launch lasts as long as its slowest state, and a thread takes
+// some 1e5 cycles for a step of one state.  Here a warp integrates one state:
 //  * lane m holds component m of every vector (state, Krylov basis, stages);
-//    dot products and norms are warp butterfly sums (every lane obtains the
-//    same bits);
+//    dot products and norms sum the lanes' products in component order, by
+//    shuffles that do not depend on one another and a chain of adds (no longer
+//    than a butterfly's five shuffle-and-add rounds), so every lane has the bits
+//    of the thread kernels' loops;
 //  * the right-hand side evaluates the reaction rates one reaction per lane
-//    (the per-reaction arithmetic of chem_source_sp), then lane k sums its
-//    species' terms in ascending reaction order from shared memory (the
-//    species-major lists t.sk_*), so the production rates equal those of the
-//    thread kernels bit for bit;
+//    (the per-reaction arithmetic of chem_source_rec or chem_source_sp), then
+//    lane k sums its species' terms in ascending reaction order from shared
+//    memory (the species-major lists t.sk_*);
 //  * the temperature Newton iteration and the 4 x 4 Krylov algebra run
 //    redundantly in every lane.
-// The dot products are summed in a different order than the sequential loops
-// of the reference (rounding-level differences).  Compiled without FMA
+// So a state gets the bits of the thread kernels.  Compiled without FMA
 // contraction, like the other chemistry kernels.
 #include <mutex>
 #include <set>
@@ -28,18 +27,22 @@
 #define WFULL 0xffffffffu
 #define WNRMAX 64          // reactions per mechanism the warp kernels take (two per lane)
 
-__device__ __forceinline__ double wsum(double x) {
+// sum_m a_m b_m over the first N lanes, in lane order
+template <int N>
+__device__ __forceinline__ double wdot(double a, double b) {
+  const double x = a * b;
+  double s = 0.0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = x + __shfl_xor_sync(WFULL, x, o);
-  return x;
+  for (int m = 0; m < N; m++) s = s + __shfl_sync(WFULL, x, m);
+  return s;
 }
 
 // Warp ROK4 of one state of NV <= 32 components (lane m holds component m;
 // lanes >= NV hold 0).  f.rhs(y, T, lane) returns the lane's component of the
 // right-hand side; f.accept / f.done as in rok4_core.
-template <int NV, class F>
-__device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, double fls, double dttry,
-                            double time_start, double time_end, int simpler, int lane) {
+template <int NV, class FN>
+__device__ void rok4_core_w(const DevCtx &c, FN &f, double &v, double T_iter, double fls, double dttry,
+                            double time_start, double time_end, int simpler, int maxsteps, int lane) {
   const double gam = 0.572816062482135;
   const double alpha[4][3] = {{0, 0, 0},
                               {0.432364435748567, 0, 0},
@@ -63,7 +66,7 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
     dt = dmin_(dt, time_end - time);
     it = it + 1;
     // ---- arnoldi (:10664-10792)
-    double rs;
+    double raw, rs;                   // f(VEC), and less fl_sav with the simpler splitting
     {
       const double TOL = 1e-6, eps = 1.0e-08;
       double HH[(STX_MMAX + 1) * STX_MMAX], HI[STX_MMAX * STX_MMAX], prj[STX_MMAX], lam[STX_MMAX];
@@ -73,10 +76,12 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
       for (int q = 0; q < STX_MMAX * STX_MMAX; q++) HI[q] = 0.0;
 #pragma unroll
       for (int q = 0; q <= STX_MMAX; q++) V[q] = 0.0;
+#pragma unroll
+      for (int q = 0; q < STX_MMAX; q++) prj[q] = 0.0;
       mA = 0;
-      rs = f.rhs(v, T_iter, lane);
-      if (simpler == 1) rs = rs - fls;
-      double nrm = sqrt(wsum(rs * rs));
+      raw = f.rhs(v, T_iter, lane);
+      rs = simpler == 1 ? raw - fls : raw;
+      double nrm = sqrt(wdot<NV>(rs, rs));
       V[0] = rs / nrm;
 #pragma unroll
       for (int kk = 1; kk <= STX_MMAX; kk++) {
@@ -85,15 +90,14 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
         jac = (jac - rs) / eps;
 #pragma unroll
         for (int jj = 1; jj <= kk; jj++) {
-          double dot = wsum(V[jj - 1] * jac);
+          double dot = wdot<NV>(V[jj - 1], jac);
           HH[(kk - 1) * (STX_MMAX + 1) + jj - 1] = dot;
           jac = jac - (dot * V[jj - 1]);
         }
-        double hn = sqrt(wsum(jac * jac));
+        double hn = sqrt(wdot<NV>(jac, jac));
         HH[(kk - 1) * (STX_MMAX + 1) + kk] = hn;
         V[kk] = jac / hn;
-#pragma unroll
-        for (int ll = 1; ll <= STX_MMAX; ll++) prj[ll - 1] = (ll <= kk) ? wsum(V[ll - 1] * rs) : 0.0;
+        prj[kk - 1] = wdot<NV>(V[kk - 1], rs);   // the earlier projections stand
 #pragma unroll
         for (int n = 1; n <= kk; n++)
 #pragma unroll
@@ -129,7 +133,7 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
       double ys = v;
 #pragma unroll
       for (int jj = 1; jj <= ii - 1; jj++) ys = ys + dt * alpha[ii - 1][jj - 1] * Ks[jj - 1];
-      double F = f.rhs(ys, T_iter, lane);
+      double F = ii == 1 ? raw : f.rhs(ys, T_iter, lane);
       double GK = 0.0;
 #pragma unroll
       for (int jj = 1; jj <= ii - 1; jj++) GK = GK + gmc[ii - 1][jj - 1] / gam * Ks[jj - 1];
@@ -138,7 +142,7 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
       double s = 0.0;
 #pragma unroll
       for (int kk = 0; kk < STX_MMAX; kk++) {
-        double pf = (kk < mA) ? wsum(V[kk] * F) : 0.0;
+        double pf = (kk < mA) ? wdot<NV>(V[kk], F) : 0.0;
         double a = vb[0] * ((kk == 0 ? 1.0 : 0.0) - inv[kk * STX_MMAX + 0]);
 #pragma unroll
         for (int jj = 1; jj < STX_MMAX; jj++) a = a + vb[jj] * ((jj == kk ? 1.0 : 0.0) - inv[kk * STX_MMAX + jj]);
@@ -153,7 +157,7 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
       b = b + dt * btv[ii] * Ks[ii];
     }
     double errv = (b - a) / ((1.0e-4) * a + 1.0e-8);
-    double errmax = sqrt(wsum(errv * errv));
+    double errmax = sqrt(wdot<NV>(errv, errv));
     double fac = 0.625 * pow(errn, 0.1) / pow(errmax, 0.175);
     double dtnext = dt * dmin_(5.0, dmax_(0.2, fac));
     if (errmax < 1.0) {
@@ -163,7 +167,7 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
     }
     dt = dtnext;
     errn = errmax;
-    if (it > c.p.ros_maxsteps) {
+    if (it > maxsteps) {
       if (lane == 0) set_status(c.p, STX_ST_ROS_STEPS_CAP);
       break;
     }
@@ -171,32 +175,45 @@ __device__ void rok4_core_w(const DevCtx &c, F &f, double &v, double T_iter, dou
   f.done(time, T_iter, it);
 }
 
-// Right-hand side of the constant-pressure reactor (cp_rhs) for the state held
-// one component per lane; returns this lane's component.  sm: per-warp shared
-// scratch of NS + WNRMAX doubles (concentrations, then the reaction rates).
-template <int NS>
-__device__ __noinline__ double cp_rhs_w(const DevCtx &c, double y, double T_iter, double h, double p, double *sm,
-                                        int lane) {
-  const DevTab &t = c.t;
-  double Yc[NS];
-#pragma unroll
-  for (int k = 0; k < NS; k++) {
-    double yk = __shfl_sync(WFULL, y, k);
-    Yc[k] = yk > 0.0 ? yk : 0.0;
-  }
-  double tt = temp_from_poly<NS>(t, t.cp, c.p, h, T_iter, Yc);
-  double rm = 0.0;
-#pragma unroll
-  for (int k = 0; k < NS; k++) rm = rm + ldg(t.rgas + k) * Yc[k];
-  double rho = p / (rm * tt);
-  double *conc = sm, *qr = sm + NS;
-  if (lane < NS) conc[lane] = rho * (y > 0.0 ? y : 0.0) / ldg(t.mw + lane);
+// Production rate of this lane's species (0 beyond NS) at T = tt from the
+// concentrations in sm[0..NS), written by the lanes just before.  sm: per-warp
+// shared scratch of NS + 1 + WNRMAX doubles (concentrations, a 1, then the
+// reaction rates).
+template <int NS, bool DD>
+__device__ __forceinline__ double production_w(const DevTab &t, double tt, double *sm, int lane) {
+  double *conc = sm, *qr = sm + NS + 1;
+  if (lane == 0) conc[NS] = 1.0;
   __syncwarp();
   const int nr = t.nr;
   double Rtti = 1.0 / (t.Ru * tt);
   int itt;
   double dtt;
   kc_pos(t, tt, itt, dtt);
+  double lh = 0.0, ll = 0.0;
+  if (DD && rec_range(t, tt)) log_dd(tt, lh, ll);
+  if (rec_range(t, tt)) {
+    for (int lr = lane; lr < nr; lr += 32) {
+      const double2 *rec = (const double2 *)t.rec + (long long)lr * (REC_N / 2);
+      const double2 c0 = __ldg(rec), c1 = __ldg(rec + 1), c2 = __ldg(rec + 2), c3 = __ldg(rec + 3);
+      const uint4 ix = __ldg((const uint4 *)(rec + 7));
+      const double *kc0 = t.kc_r + (long long)(itt - 1) * nr + lr;
+      const double ka = ldg(kc0), kc = ka + (ldg(kc0 + nr) - ka) * dtt;
+      const int fl = __double2loint(c3.y), cls = fl & 255;
+      double tbs = 1.0;
+      if (cls != REC_PLAIN) {
+        tbs = 0.0;
+        const double *ef = t.rec_eff + (long long)lr * t.rec_es;
+#pragma unroll
+        for (int k = 0; k < NS; k++) tbs = tbs + ldg(ef + k) * conc[k];
+      }
+      const double kf = rec_kf<DD>(t, lr, cls, c0, c1, c2, c3.x, tt, Rtti, lh, ll, tbs);
+      const double kb = (fl >> 8) & 255 ? kf / kc : 0.0;
+      const double q1 = conc[ix.x & 255] * conc[(ix.x >> 8) & 255] * conc[(ix.x >> 16) & 255];
+      const double q2 = conc[ix.x >> 24] * conc[ix.y & 255] * conc[(ix.y >> 8) & 255];
+      const double tb = cls == REC_TB ? tbs : 1.0;
+      qr[lr] = tb * (kf * q1 - kb * q2);
+    }
+  } else {
   for (int lr = lane; lr < nr; lr += 32) {
     int ty = __ldg(t.reac_ty + lr);
     double tbs = 1.0;
@@ -226,6 +243,7 @@ __device__ __noinline__ double cp_rhs_w(const DevCtx &c, double y, double T_iter
     double tb = (ty == 1) ? tbs : 1.0;
     qr[lr] = tb * (kf * q1 - kb * q2);
   }
+  }
   __syncwarp();
   double acc = 0.0;
   if (lane < NS) {
@@ -238,7 +256,150 @@ __device__ __noinline__ double cp_rhs_w(const DevCtx &c, double y, double T_iter
     }
   }
   __syncwarp();
+  return acc;
+}
+
+// Right-hand side of the constant-pressure reactor (cp_rhs) for the state held
+// one component per lane; returns this lane's component.
+template <int NS>
+__device__ __noinline__ double cp_rhs_w(const DevCtx &c, double y, double T_iter, double h, double p, double *sm,
+                                        int lane) {
+  const DevTab &t = c.t;
+  double Yc[NS];
+#pragma unroll
+  for (int k = 0; k < NS; k++) {
+    double yk = __shfl_sync(WFULL, y, k);
+    Yc[k] = yk > 0.0 ? yk : 0.0;
+  }
+  double tt = temp_from_poly<NS>(t, t.cp, c.p, h, T_iter, Yc);
+  double rm = 0.0;
+#pragma unroll
+  for (int k = 0; k < NS; k++) rm = rm + ldg(t.rgas + k) * Yc[k];
+  double rho = p / (rm * tt);
+  if (lane < NS) sm[lane] = rho * (y > 0.0 ? y : 0.0) / ldg(t.mw + lane);
+  const double acc = production_w<NS, true>(t, tt, sm, lane);
   return lane < NS ? acc / rho : 0.0;
+}
+
+// Right-hand side of a flow cell (krylov_rhs), the species densities one per
+// lane; m0..m3 the momentum components and the energy.  Lanes beyond NS return 0.
+template <int NS, bool DD>
+__device__ __noinline__ double flow_rhs_w(const DevCtx &c, double y, double m0, double m1, double m2, double m3,
+                                          double T_iter, double *sm, int lane) {
+  const DevTab &t = c.t;
+  const double yc = y > 0.0 ? y : 0.0;
+  double Y[NS];
+#pragma unroll
+  for (int k = 0; k < NS; k++) Y[k] = __shfl_sync(WFULL, yc, k);
+  double rho = Y[0];
+#pragma unroll
+  for (int k = 1; k < NS; k++) rho = rho + Y[k];
+  const double ri = 1.0 / rho;
+#pragma unroll
+  for (int k = 0; k < NS; k++) Y[k] = Y[k] * ri;
+  if (lane < NS) sm[lane] = rho * (yc * ri) / ldg(t.mw + lane);
+  const double uu = m0 * ri, vv = m1 * ri, ww = m2 * ri;
+  const double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
+  const double ee = (m3 * ri) - qq;
+  const double tt = temp_from_e<NS>(t, c.p, ee, T_iter, Y);
+  return production_w<NS, DD>(t, tt, sm, lane);
+}
+
+// The flow cell, one component per lane.  FULL: the state is (rho Y_k, rho u,
+// rho v, rho w, rho E) as in Rok4Flow; otherwise the species densities alone, the
+// other four fixed in mom, as in Rok4FlowSpecies.
+template <int NS, bool FULL>
+struct Rok4FlowW {
+  const DevCtx &c;
+  double mom[4];
+  double *sm;
+  __device__ __forceinline__ double rhs(double y, double T_iter, int lane) const {
+    double m[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) m[q] = FULL ? __shfl_sync(WFULL, y, NS + q) : mom[q];
+    return flow_rhs_w<NS, !FULL>(c, y, m[0], m[1], m[2], m[3], T_iter, sm, lane);
+  }
+  __device__ __forceinline__ void accept(double v, double, double &T_iter, double &, int) const {
+    double Y[NS], m[4];
+#pragma unroll
+    for (int k = 0; k < NS; k++) Y[k] = __shfl_sync(WFULL, v, k);
+#pragma unroll
+    for (int q = 0; q < 4; q++) m[q] = FULL ? __shfl_sync(WFULL, v, NS + q) : mom[q];
+    double rho = Y[0];
+#pragma unroll
+    for (int k = 1; k < NS; k++) rho = rho + Y[k];
+    const double ri = 1.0 / rho;
+#pragma unroll
+    for (int k = 0; k < NS; k++) Y[k] = Y[k] * ri;
+    const double uu = m[0] * ri, vv = m[1] * ri, ww = m[2] * ri;
+    const double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
+    const double ee = m[3] * ri - qq;
+    T_iter = temp_from_e<NS>(c.t, c.p, ee, T_iter, Y);
+  }
+  __device__ __forceinline__ void done(double, double, int) const {}
+};
+
+// One warp per flow cell (k_rok4's work on a small grid).
+template <int NS>
+__global__ void __launch_bounds__(128, 4)
+    k_rok4_w(DevCtx c, const DevCtx *__restrict__ cg, double *__restrict__ w, const double *__restrict__ wa,
+             const double *__restrict__ fl_sav, double dttry, double t0, double t1, int simpler) {
+  __shared__ double sm_all[4][NS + 1 + WNRMAX];
+  const DevGrid &g = c.g;
+  const double eps_Z = 5e-4;
+  if (c.p.dt_d) dttry = dttry * *c.p.dt_d;   // captured CFL-driven step: dttry holds the splitting's factor
+  if (c.p.time_d) {                 // captured step: the window starts at the device-held time
+    t0 = *c.p.time_d;
+    t1 = t0 + dttry;
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long cell = (long long)blockIdx.x * 4 + wid;
+  if (cell >= g.npi) return;
+  const int i = 1 + (int)(cell % g.nx);
+  const long long r = cell / g.nx;
+  const int j = 1 + (int)(r % g.ny), k = 1 + (int)(r / g.ny);
+  const long long p = gidx(g, i, j, k);
+  const double Z = FG(wa, p, NS + 12);
+  if (!(Z > eps_Z && Z < 1.0 - eps_Z)) return;
+  const double T = FG(wa, p, NS + 5);
+  double v = lane < NS + 4 ? FG(w, p, lane + 1) : 0.0;
+  const int maxsteps = cg->p.ros_maxsteps;
+  if (simpler != 1) {
+    Rok4FlowW<NS, false> f{*cg, {}, sm_all[wid]};
+#pragma unroll
+    for (int q = 0; q < 4; q++) f.mom[q] = __shfl_sync(WFULL, v, NS + q);
+    v = lane < NS ? v : 0.0;
+    rok4_core_w<NS>(*cg, f, v, T, 0.0, dttry, t0, t1, 0, maxsteps, lane);
+    if (lane < NS) FG(w, p, lane + 1) = v;
+  } else {
+    Rok4FlowW<NS, true> f{*cg, {}, sm_all[wid]};
+    const double fls = lane < NS + 4 ? fl_sav[cell + (long long)lane * g.npi] : 0.0;
+    rok4_core_w<NS + 4>(*cg, f, v, T, fls, dttry, t0, t1, 1, maxsteps, lane);
+    if (lane < NS + 4) FG(w, p, lane + 1) = v;
+  }
+}
+
+template <int NS>
+static int rok4_w_t(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa,
+                    const double *fl_sav, double dttry, double t0, double t1, int simpler) {
+  if constexpr (NS + 4 > 32) {
+    return STX_E_UNSUPPORTED;
+  } else {
+    if (c.t.nr > WNRMAX) return STX_E_UNSUPPORTED;
+    k_rok4_w<NS><<<(unsigned)((c.g.npi + 3) / 4), 128, 0, s>>>(c, cg, w, wa, fl_sav, dttry, t0, t1, simpler);
+    STX_CUDA_TRY(cudaGetLastError());
+    return STX_OK;
+  }
+}
+
+int launch_rok4_warp(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa,
+                     const double *fl_sav, double dttry, double t0, double t1, int simpler) {
+  switch (c.t.ns) {
+#define X(N) case N: return rok4_w_t<N>(c, cg, s, w, wa, fl_sav, dttry, t0, t1, simpler);
+    STX_FOR_NS(X)
+#undef X
+    default: return STX_E_UNSUPPORTED;
+  }
 }
 
 template <int NS>
@@ -280,7 +441,7 @@ __global__ void __launch_bounds__(128) k_batch0d_w(DevCtx c, int n, const double
                                                    double *__restrict__ Y, double *__restrict__ T,
                                                    double *__restrict__ t_ign, double *__restrict__ t_end,
                                                    int *__restrict__ nsteps, unsigned int *counter) {
-  __shared__ double sm_all[4][NS + WNRMAX];
+  __shared__ double sm_all[4][NS + 1 + WNRMAX];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double *sm = sm_all[wid];
   for (;;) {
@@ -294,7 +455,7 @@ __global__ void __launch_bounds__(128) k_batch0d_w(DevCtx c, int n, const double
 #pragma unroll 1
     for (int k = 0; k < NS; k++) h = h + Y0[(long long)k * n + r] * species_poly_int(c.t, c.t.cpi, T0r, k + 1);
     Rok4ConstPW<NS> f{c, h, p0[r], T0r, ign_factor, end_factor, sm, -1.0, 0.0, T0r, 0};
-    rok4_core_w<NS>(c, f, v, T0r, 0.0, dttry, 0.0, t_max, 0, lane);
+    rok4_core_w<NS>(c, f, v, T0r, 0.0, dttry, 0.0, t_max, 0, c.p.ros_maxsteps, lane);
     if (lane < NS) Y[(long long)lane * n + r] = v;
     if (lane == 0) {
       T[r] = f.T_final;

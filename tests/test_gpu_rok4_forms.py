@@ -1,0 +1,99 @@
+"""The forms of the ROK4 cell update against one another.
+
+A grid of up to 8192 cells takes a warp per cell and a larger one a thread per
+cell, with the same operations in the same order: the same cells give the same
+bits.  A mechanism whose reactions all fit the packed records takes them;
+otherwise the sparse stoichiometry lists serve it.  Both are run on the same
+cells: without the Strang splitting's shared exponential the bits are the same,
+with it the rates differ by rounding.
+"""
+import ctypes as C
+import dataclasses
+
+import numpy as np
+import pytest
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+from stx import case as CS  # noqa: E402
+from stx.native import check  # noqa: E402
+from stx.solver import Solver  # noqa: E402
+
+DT = 2e-7
+
+
+def _source(case, simpler, seed=7):
+    """A prepared solver and its fl_sav (the simpler splitting's residual)."""
+    s = Solver(case)
+    s.update_ghost(1)
+    s.compute_aux(1, 1)
+    rng = np.random.default_rng(seed)
+    scale = np.abs(case.interior(s.host_w())).max(axis=(1, 2, 3)) * 1e3
+    fs = torch.from_numpy(rng.standard_normal(tuple(s.fl_sav.shape)) * scale[:, None, None, None]).to(s.device)
+    return s, fs if simpler else None
+
+
+def _rok4(s, fs, simpler):
+    check(s.lib.stx_rosenbrock_krylov(s.ctx, s.stream, C.c_void_p(s.w.data_ptr()), C.c_void_p(s.w_aux.data_ptr()),
+                                      None if fs is None else C.c_void_p(fs.data_ptr()), DT, 0.0, DT, simpler), "rok4")
+    torch.cuda.synchronize()
+    return s.case.interior(s.host_w())
+
+
+@pytest.mark.parametrize("n", [(16, 16, 8), (13, 9, 7), (32, 16, 16)])
+@pytest.mark.parametrize("simpler", [0, 1])
+def test_warp_per_cell_equals_thread_per_cell(n, simpler):
+    """A small box, and the same box repeated until the thread-per-cell kernel takes it."""
+    small = H.synthetic_case(n=n, seed=31, T0=1300.0, amp_T=400.0)
+    s, fs = _source(small, simpler)
+    rep = -(-8193 // (n[0] * n[1] * n[2]))
+    big = H.synthetic_case(n=(n[0], n[1], n[2] * rep), seed=31, T0=1300.0, amp_T=400.0)
+    b = Solver(big)
+    b.compute_aux(1, 1)
+    for src, dst in ((s.w, b.w), (s.w_aux, b.w_aux)):
+        big.interior(dst)[:] = small.interior(src).repeat(1, rep, 1, 1)
+    fb = None if fs is None else fs.repeat(1, rep, 1, 1).contiguous()
+    got, ref = _rok4(s, fs, simpler), _rok4(b, fb, simpler)
+    for q in range(rep):
+        assert np.array_equal(got, ref[:, q * n[2]:(q + 1) * n[2]]), q
+    s.close()
+    b.close()
+
+
+def _padded(case):
+    """The case with one more, inert reaction (A = 0) whose stoichiometry fits no record."""
+    tb = case.tb
+    row = lambda a, v: np.concatenate([a, np.full((1,) + a.shape[1:], v, a.dtype)])
+    rc, pc = row(tb.r_coeffs, 0), row(tb.p_coeffs, 0)
+    rc[-1, 0], pc[-1, 1] = 1.5, 1.5
+    tb = dataclasses.replace(tb, nr=tb.nr + 1, reac_ty=row(tb.reac_ty, 0), is_rev=row(tb.is_rev, 0),
+                             arr_a=row(tb.arr_a, 0), arr_b=row(tb.arr_b, 0), arr_ea=row(tb.arr_ea, 0),
+                             falloff=row(tb.falloff, 0), tb_eff=row(tb.tb_eff, 0), r_coeffs=rc, p_coeffs=pc,
+                             kc_tab=np.concatenate([tb.kc_tab, np.ones_like(tb.kc_tab[:, :1])], axis=1))
+    return CS.Case(case.cfg, tb)
+
+
+@pytest.mark.parametrize("n", [(8, 6, 5), (32, 20, 16)])
+@pytest.mark.parametrize("simpler", [0, 1])
+def test_records_equal_sparse_lists(n, simpler):
+    case = H.synthetic_case(n=n, seed=33, T0=1300.0, amp_T=400.0)
+    other = _padded(case)
+    other.w[:], other.w_aux[:] = case.w, case.w_aux
+    (s, fs), (o, fo) = _source(case, simpler), _source(other, simpler)
+    got, ref = _rok4(s, fs, simpler), _rok4(o, fo, simpler)
+    if simpler:
+        assert np.array_equal(got, ref)
+    else:
+        # A rounding of the rates, 1e-16, enters the finite-difference Jacobian
+        # divided by its step of 1e-8, and an adaptive window carries that: 1e-8
+        # of the species' scale.
+        for m in range(case.nv):
+            H.assert_close(got[m], ref[m], 1e-8, f"w[{m}]", floor=np.abs(ref[m]).max())
+    s.close()
+    o.close()
