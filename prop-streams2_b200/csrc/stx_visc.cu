@@ -22,6 +22,26 @@
 #define STX_VISC_MINB 5
 #endif
 
+// Species enthalpy (get_species_h_from_temperature_dev).  In the two-range form
+// the range comes from one comparison per point (hi, mid_mask) instead of a
+// search per species whose table loads the coefficient loads wait for, and a
+// row is three 16-byte loads.  The same terms in the same order as
+// species_poly_int.  Measured on a B200: all five flux calls on a 150 x 101 x 77
+// box 5.27 -> 4.21 ms; a step of the 256^3 turbulence box 225 -> 206 ms.
+template <int NS>
+__device__ __forceinline__ double enthalpy(const DevTab &t, double tt, int k, unsigned long long hi) {
+  if (!t.poly2) return species_poly_int(t, t.cpi, tt, k + 1);
+  const bool up = t.umid >= 0.0 ? hi != 0 : (hi >> k) & 1ull;
+  const double2 *b = (const double2 *)(t.cpi6 + k * 6 + (up ? NS * 6 : 0));
+  const double2 u = __ldg(b), v = __ldg(b + 1), x = __ldg(b + 2);
+  const double t2 = tt * tt, t3 = t2 * tt, t4 = t3 * tt, t5 = t4 * tt;
+  double hh = x.y + u.x * tt;
+  hh = hh + u.y * t2;
+  hh = hh + v.x * t3;
+  hh = hh + v.y * t4;
+  return hh + x.x * t5;
+}
+
 // One staggered face between points p (left) and q = p + st (right), computed in
 // R (double: plain form; float: mixed form, fields rounded once on load).  hl
 // carries the species enthalpies at
@@ -69,14 +89,16 @@ __device__ __forceinline__ void visc_face(const DevCtx &c, const double *__restr
   }
   fhat_tmp = fhat_tmp * mwmif;
   R et = R(0.0);
+  const unsigned long long hi = t.poly2 ? mid_mask<NS>(t, (double)ttp) : 0ull;
+  const unsigned long long hi0 = t.poly2 && !have_hl ? mid_mask<NS>(t, (double)tt) : 0ull;
 #pragma unroll
   for (int k = 0; k < NS; k++) {
     R yyf = R(0.5) * (yp[k] + yl[k]);
     R xxp = yp[k] * mwmp, xx = yl[k] * mwm;
     R sig = -rd[k] * (xxp - xx) * mwmif + fhat_tmp * yyf;
     fh[k] = sig;
-    R hh = have_hl ? hl[k] : (R)species_poly_int(t, t.cpi, (double)tt, k + 1);
-    R hhp = (R)species_poly_int(t, t.cpi, (double)ttp, k + 1);
+    R hh = have_hl ? hl[k] : (R)enthalpy<NS>(t, (double)tt, k, hi0);
+    R hhp = (R)enthalpy<NS>(t, (double)ttp, k, hi);
     hl[k] = hhp;
     R hhf = R(0.5) * (hh + hhp);
     et = et + sig * hhf;
