@@ -19,7 +19,11 @@
 #endif
 
 // Grids of at most this many cells take a warp per cell (k_rok4_w): the bits are
-// the same, and a thread per cell leaves most of the chip idle there.
+// the same, and a thread per cell leaves most of the chip idle there.  One 2e-8 s
+// window of H2/air cells on a B200, thread against warp: 1024 cells 791 / 193 us,
+// 4096 814 / 309, 8192 811 / 548, 12288 825 / 760, 16384 825 / 986 (simpler
+// splitting 1033 / 227, 1052 / 362, 1055 / 652, 1066 / 919, 1065 / 1184).  The lines
+// cross near 13000; cells that need more steps move it, hence the margin.
 #ifndef STX_ROK4_WARP_CELLS
 #define STX_ROK4_WARP_CELLS 8192
 #endif
