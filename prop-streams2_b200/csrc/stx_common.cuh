@@ -381,7 +381,8 @@ __device__ double temp_from_poly(const DevTab &t, const double *coef, const DevP
 // quotient the reference forms for every term, formed once at context creation
 // (the same correctly rounded division, so the same bits).  The powers T^(l+1)
 // for l + 1 >= 1 are formed incrementally, T^(n+1) = T^n * T, the very products
-// of the repeated multiplication ipow performs.
+// of the repeated multiplication ipow performs.  Products and sums are rounded
+// one by one in every file, also where FMA contraction is on.
 __device__ __forceinline__ double species_poly_int(const DevTab &t, const double *ai, double tt, int isp) {
   int nr = 1;
   if (t.nset > 1) nr = locate_range(t, tt, isp);
@@ -390,12 +391,12 @@ __device__ __forceinline__ double species_poly_int(const DevTab &t, const double
   int tpe = 0;
   for (int l = t.icl; l <= t.icr; l++) {
     if (l == -1) {
-      hh = hh + cpc(t, ai, l, isp, nr) * log(tt);
+      hh = __dadd_rn(hh, __dmul_rn(cpc(t, ai, l, isp, nr), log(tt)));
     } else if (l + 1 >= 1) {
       while (tpe < l + 1) { tp = tp * tt; tpe++; }
-      hh = hh + cpc(t, ai, l, isp, nr) * tp;
+      hh = __dadd_rn(hh, __dmul_rn(cpc(t, ai, l, isp, nr), tp));
     } else {
-      hh = hh + cpc(t, ai, l, isp, nr) * ipow(tt, l + 1);
+      hh = __dadd_rn(hh, __dmul_rn(cpc(t, ai, l, isp, nr), ipow(tt, l + 1)));
     }
   }
   return hh;

@@ -22,12 +22,20 @@
 #define STX_VISC_MINB 5
 #endif
 
+// The roundings of a face flux are written out (fma and mul_rn; the compiler
+// contracts neither further): where two products meet, which of them it contracts
+// depends on the code around them, and the captured flame of 2000 cells turns a
+// last bit of the energy flux into 8e-6 of its species within a few ROK4 windows.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+
 // Species enthalpy (get_species_h_from_temperature_dev).  In the two-range form
 // the range comes from one comparison per point (hi, mid_mask) instead of a
 // search per species whose table loads the coefficient loads wait for, and a
-// row is three 16-byte loads.  The same terms in the same order as
-// species_poly_int.  Measured on a B200: all five flux calls on a 150 x 101 x 77
-// box 5.27 -> 4.21 ms; a step of the 256^3 turbulence box 225 -> 206 ms.
+// row is three 16-byte loads.  The same terms in the same order and with the same
+// roundings as species_poly_int.  Measured on a B200: all five flux calls on a
+// 150 x 101 x 77 box 5.27 -> 4.24 ms (4.24 with contracted products too); a step of
+// the 256^3 turbulence box 225 -> 206 ms.
 template <int NS>
 __device__ __forceinline__ double enthalpy(const DevTab &t, double tt, int k, unsigned long long hi) {
   if (!t.poly2) return species_poly_int(t, t.cpi, tt, k + 1);
@@ -35,11 +43,11 @@ __device__ __forceinline__ double enthalpy(const DevTab &t, double tt, int k, un
   const double2 *b = (const double2 *)(t.cpi6 + k * 6 + (up ? NS * 6 : 0));
   const double2 u = __ldg(b), v = __ldg(b + 1), x = __ldg(b + 2);
   const double t2 = tt * tt, t3 = t2 * tt, t4 = t3 * tt, t5 = t4 * tt;
-  double hh = x.y + u.x * tt;
-  hh = hh + u.y * t2;
-  hh = hh + v.x * t3;
-  hh = hh + v.y * t4;
-  return hh + x.x * t5;
+  double hh = __dadd_rn(x.y, mul_rn(u.x, tt));
+  hh = __dadd_rn(hh, mul_rn(u.y, t2));
+  hh = __dadd_rn(hh, mul_rn(v.x, t3));
+  hh = __dadd_rn(hh, mul_rn(v.y, t4));
+  return __dadd_rn(hh, mul_rn(x.x, t5));
 }
 
 // One staggered face between points p (left) and q = p + st (right), computed in
@@ -56,8 +64,8 @@ __device__ __forceinline__ void visc_face(const DevCtx &c, const double *__restr
   R uu = ld(p, J_U), uup = ld(q, J_U), vv = ld(p, J_V), vvp = ld(q, J_V);
   R ww = ld(p, J_W), wwp = ld(q, J_W), tt = ld(p, J_T), ttp = ld(q, J_T);
   R mu = ld(p, J_MU), mup = ld(q, J_MU), kc = ld(p, J_K), kcp = ld(q, J_K);
-  R qq = R(0.5) * (uu * uu + vv * vv + ww * ww);
-  R qqp = R(0.5) * (uup * uup + vvp * vvp + wwp * wwp);
+  R qq = R(0.5) * fma(ww, ww, fma(uu, uu, mul_rn(vv, vv)));
+  R qqp = R(0.5) * fma(wwp, wwp, fma(uup, uup, mul_rn(vvp, vvp)));
   R sigx = uup - uu, sigy = vvp - vv, sigz = wwp - ww;
   R sigq_tt = ttp - tt, sigq_qq = qqp - qq;
   R muf = mu + mup;
@@ -65,7 +73,7 @@ __device__ __forceinline__ void visc_face(const DevCtx &c, const double *__restr
   R kf = kc + kcp;
   kf = R(0.5) * kf / dxf;
   sigx = sigx * muf; sigy = sigy * muf; sigz = sigz * muf;
-  R sigq = sigq_tt * kf + sigq_qq * muf;
+  R sigq = fma(sigq_qq, muf, mul_rn(sigq_tt, kf));
   R yl[NS], yp[NS];
 #pragma unroll
   for (int k = 0; k < NS; k++) { yl[k] = ld(p, k + 1); yp[k] = ld(q, k + 1); }
@@ -84,8 +92,8 @@ __device__ __forceinline__ void visc_face(const DevCtx &c, const double *__restr
 #pragma unroll
   for (int k = 0; k < NS; k++) {
     rd[k] = R(0.5) * (ld(p, J_D + 1 + k) + ld(q, J_D + 1 + k));
-    R xxp = yp[k] * mwmp, xx = yl[k] * mwm;
-    fhat_tmp = fhat_tmp + (xxp - xx) * rd[k];
+    const R dx = fma(yp[k], mwmp, -mul_rn(yl[k], mwm));
+    fhat_tmp = fma(dx, rd[k], fhat_tmp);
   }
   fhat_tmp = fhat_tmp * mwmif;
   R et = R(0.0);
@@ -94,14 +102,14 @@ __device__ __forceinline__ void visc_face(const DevCtx &c, const double *__restr
 #pragma unroll
   for (int k = 0; k < NS; k++) {
     R yyf = R(0.5) * (yp[k] + yl[k]);
-    R xxp = yp[k] * mwmp, xx = yl[k] * mwm;
-    R sig = -rd[k] * (xxp - xx) * mwmif + fhat_tmp * yyf;
+    const R dx = fma(yp[k], mwmp, -mul_rn(yl[k], mwm));
+    R sig = fma(fhat_tmp, yyf, mul_rn(-rd[k] * dx, mwmif));
     fh[k] = sig;
     R hh = have_hl ? hl[k] : (R)enthalpy<NS>(t, (double)tt, k, hi0);
     R hhp = (R)enthalpy<NS>(t, (double)ttp, k, hi);
     hl[k] = hhp;
     R hhf = R(0.5) * (hh + hhp);
-    et = et + sig * hhf;
+    et = fma(sig, hhf, et);
   }
   fh[NS] = -sigx;
   fh[NS + 1] = -sigy;
