@@ -331,15 +331,18 @@ typedef struct stx_tuning {
   int32_t sweep_kind[3];     /* convective sweep x, y, z: 0 staged shared-memory tiles, 1 one face per thread */
   int32_t weno_list[3];      /* 1: the faces the Ducros sensor marks are listed and computed by full warps;
                                 0: computed in line by the sweep */
-  int32_t chem_ctas_per_sm;  /* persistent CTAs per SM of the cell chemistry (ROK4); 0: its occupancy limit;
-                                -1: the plain launch, one thread per cell and no work stealing (the
-                                same per-cell arithmetic: the results are the same bit for bit) */
+  int32_t chem_ctas_per_sm;  /* cell chemistry (ROK4): persistent CTAs per SM of the thread-per-cell kernel;
+                                -1: its plain launch, one thread per cell and no work stealing; 0: chosen
+                                by size, a warp per cell on small grids (up to 8192 cells, up to 28 species
+                                and 64 reactions), else the occupancy limit (the same per-cell arithmetic:
+                                the results are the same bit for bit) */
   int32_t chem_ctas_max;     /* out: that occupancy limit */
   int32_t batch_ctas_max;    /* most CTAs of one stx_batch0d_integrate launch; 0: no cap (a server running
                                 several reactor launches at once caps each, leaving room for other work) */
   float sweep_ms[3];         /* out (stx_autotune): time of the chosen sweep kernels, ms */
   float chem_ms;             /* out (stx_autotune): time of the chosen chemistry launch, ms (stx_autotune tries
-                                the persistent CTA counts from the limit down, then the plain launch) */
+                                the warp per cell where 0 takes it, the persistent CTA counts from the limit
+                                down, then the plain launch) */
 } stx_tuning;
 int stx_get_tuning(stx_ctx *ctx, stx_tuning *out);
 int stx_set_tuning(stx_ctx *ctx, const stx_tuning *t);

@@ -1154,19 +1154,24 @@ int stx_autotune(stx_ctx *c, void *sv, const stx_fields *f, double dt_chem, stx_
     c->weno_list[d] = pick.list;
     sweep_ms[d] = best;
   }
-  // ---- cell chemistry (ROK4), on a scratch copy of w: persistent CTAs per SM
-  // (work stealing), then the plain launch (one thread per cell, -1), which the
-  // hardware's block scheduler balances instead
+  // ---- cell chemistry (ROK4), on a scratch copy of w: a warp per cell where that
+  // is the default (0), persistent CTAs per SM (work stealing), then the plain
+  // launch (one thread per cell, -1), which the hardware's block scheduler balances
+  // instead
   const stx_params &p = c->par;
   if (rc == STX_OK && p.enable_chemistry == 2 && p.rosenbrock_version == 2 && dt_chem > 0.0) {
     if (cudaMallocFromPoolAsync((void **)&w2, nw * sizeof(double), pool, s) != cudaSuccess) {
       rc = STX_E_NOMEM;
     } else {
       const int lim = chem_ctas_limit(c->ns);
+      const bool warp = rok4_takes_warp(c->d.t, g.npi);
+      std::vector<int> cands;                              // the default first
+      if (warp) cands.push_back(0);
+      for (int k = lim; k >= -1; k--)
+        if (k != 0) cands.push_back(k);
       float best = -1.f;
       int pick = 0;
-      for (int k = lim; k >= -1 && rc == STX_OK; k--) {    // the default (the limit) first
-        if (k == 0) continue;
+      for (int k : cands) {
         c->d.p.chem_ctas_per_sm = k;
         float ms = time_launches(s, e0, e1, 1, [&] {
           if (cudaMemcpyAsync(w2, f->w, nw * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -1176,7 +1181,7 @@ int stx_autotune(stx_ctx *c, void *sv, const stx_fields *f, double dt_chem, stx_
         if (ms < 0.f) { rc = STX_E_CUDA; break; }
         if (best < 0.f || ms < 0.95f * best) { best = ms; pick = k; }
       }
-      c->d.p.chem_ctas_per_sm = pick == lim ? 0 : pick;
+      c->d.p.chem_ctas_per_sm = !warp && pick == lim ? 0 : pick;
       chem_ms = best;
     }
   }

@@ -18,7 +18,8 @@
 #define STX_ROK4_MINB 4
 #endif
 
-// Grids of at most this many cells take a warp per cell (k_rok4_w): the bits are
+// Grids of at most this many cells take a warp per cell (k_rok4_w) unless the
+// context names a launch of the thread-per-cell kernel (stx_tuning): the bits are
 // the same, and a thread per cell leaves most of the chip idle there.  One 2e-8 s
 // window of H2/air cells on a B200, thread against warp: 1024 cells 791 / 193 us,
 // 4096 814 / 309, 8192 811 / 548, 12288 825 / 760, 16384 825 / 986 (simpler
@@ -377,13 +378,13 @@ int chem_ctas_limit(int ns) {
   return per < 1 ? 1 : per;
 }
 
+bool rok4_takes_warp(const DevTab &t, long long npi) { return npi <= STX_ROK4_WARP_CELLS && rok4_warp_serves(t); }
+
 template <int NS>
 static int rok4_t(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa, const double *fl_sav,
                   double dttry, double t0, double t1, int simpler, unsigned int *counter) {
-  if (c.g.npi <= STX_ROK4_WARP_CELLS) {
-    int rc = launch_rok4_warp(c, cg, s, w, wa, fl_sav, dttry, t0, t1, simpler);
-    if (rc != STX_E_UNSUPPORTED) return rc;
-  }
+  if (c.p.chem_ctas_per_sm == 0 && rok4_takes_warp(c.t, c.g.npi))
+    return launch_rok4_warp(c, cg, s, w, wa, fl_sav, dttry, t0, t1, simpler);
   long long need = (c.g.npi + chem_block(NS) - 1) / chem_block(NS);
   if (c.p.chem_ctas_per_sm < 0) {            // the plain launch: a thread per cell, no work stealing
     k_rok4<NS><<<(unsigned)need, chem_block(NS), 0, s>>>(c, cg, w, wa, fl_sav, dttry, t0, t1, simpler, nullptr);

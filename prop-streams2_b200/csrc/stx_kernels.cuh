@@ -57,7 +57,9 @@ int chem_ctas_limit(int ns);
 // cg: the device-resident copy of c (stx_ctx::dctx_d)
 int launch_rok4(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa, const double *fl_sav,
                 double dttry, double t0, double t1, int simpler, unsigned int *counter);
-// the same with a warp per cell, for small grids (STX_E_UNSUPPORTED: not for this mechanism)
+// whether a context whose tuning leaves the chemistry's launch open takes a warp per cell
+bool rok4_takes_warp(const DevTab &t, long long npi);
+bool rok4_warp_serves(const DevTab &t);   // whether the warp kernel has this mechanism
 int launch_rok4_warp(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa,
                      const double *fl_sav, double dttry, double t0, double t1, int simpler);
 int launch_rosenbrock(const DevCtx &c, cudaStream_t s, double *w, double *wa, double dttry, double t0, double t1,

@@ -395,6 +395,15 @@ static int rok4_w_t(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w
   }
 }
 
+bool rok4_warp_serves(const DevTab &t) {
+  switch (t.ns) {
+#define X(N) case N: return N + 4 <= 32 && t.nr <= WNRMAX;
+    STX_FOR_NS(X)
+#undef X
+    default: return false;
+  }
+}
+
 int launch_rok4_warp(const DevCtx &c, const DevCtx *cg, cudaStream_t s, double *w, const double *wa,
                      const double *fl_sav, double dttry, double t0, double t1, int simpler) {
   switch (c.t.ns) {
