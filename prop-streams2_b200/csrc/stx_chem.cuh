@@ -390,10 +390,11 @@ __device__ __forceinline__ void chem_source_rows(const DevTab &t, double tt, dou
 // rosenbrock_krylov_rhs (kernels_gpu.F90:10794-10976), PaSR off.  With the
 // context's tables (KCF false) the production terms run over the sparse
 // stoichiometry with per-thread rows in shared memory (launch with
-// chem_block(NS) threads); with the reference's raw tables (KCF true) over the
-// dense species loops.
-template <int NS, bool KCF = false, bool DD = false>
-__device__ STX_RHS_LINKAGE void krylov_rhs(const DevCtx &c, const double *w_sav, const double *w_mom, double T_iter,
+// chem_block(NS) threads); with the reference's raw tables (KCF true), which have
+// neither records nor the two-range form, over the dense species loops.
+// CTX: DevCtx, or a caller's own context with the tables t and the parameters p.
+template <int NS, bool KCF = false, bool DD = false, class CTX>
+__device__ STX_RHS_LINKAGE void krylov_rhs(const CTX &c, const double *w_sav, const double *w_mom, double T_iter,
                                            double *rhs) {
   const DevTab &t = c.t;
   double Y[NS], conc[NS], wl[NS];
@@ -411,7 +412,7 @@ __device__ STX_RHS_LINKAGE void krylov_rhs(const DevCtx &c, const double *w_sav,
   double uu = w_mom[0] * ri, vv = w_mom[1] * ri, ww = w_mom[2] * ri;
   double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
   double ee = (w_mom[3] * ri) - qq;
-  double tt = temp_from_e<NS>(t, c.p, ee, T_iter, Y);
+  double tt = temp_from_e<NS, !KCF>(t, c.p, ee, T_iter, Y);
   if (KCF) {
 #pragma unroll
     for (int m = 0; m < NS; m++) rhs[m] = 0.0;
@@ -545,8 +546,8 @@ __constant__ double c_rok4_bt[STX_NSTAGE] = {-0.217819895945721, 1.0313084747846
 // finite-difference Jacobian products, the small Krylov matrices and the error
 // norm stay FP64 and only those two arrays are rounded to FP32.  f(VEC), which
 // the finite differences subtract, is then kept in the FP64 scratch S2.
-template <int NV, class F, typename A = double>
-__device__ void rok4_core(const DevCtx &c, F &f, double *VEC, double T_iter, const double *fls, long long fstride,
+template <int NV, class F, typename A = double, class CTX>
+__device__ void rok4_core(const CTX &c, F &f, double *VEC, double T_iter, const double *fls, long long fstride,
                           double dttry, double time_start, double time_end, int simpler, int maxsteps) {
   const double gam = 0.572816062482135;
   constexpr bool AD = std::is_same<A, double>::value;
@@ -732,9 +733,9 @@ __device__ void rok4_core(const DevCtx &c, F &f, double *VEC, double T_iter, con
 // The flow cell: state (rho Y_k, rho u, rho v, rho w, rho E), constant volume
 // (rosenbrock_krylov_rhs, :10794-10976); after an accepted step T follows from
 // e by the Newton inversion (:10597-10606).
-template <int NS, bool KCF>
+template <int NS, bool KCF, class CTX = DevCtx>
 struct Rok4Flow {
-  const DevCtx &c;
+  const CTX &c;
   __device__ __forceinline__ void rhs(const double *y, double T_iter, double *out) const {
     krylov_rhs<NS, KCF>(c, y, y + NS, T_iter, out);
 #pragma unroll
@@ -749,7 +750,7 @@ struct Rok4Flow {
     double uu = VEC[NS] * ri, vv = VEC[NS + 1] * ri, ww = VEC[NS + 2] * ri;
     double qq = 0.5 * (uu * uu + vv * vv + ww * ww);
     double ee = VEC[NS + 3] * ri - qq;
-    T_iter = temp_from_e<NS>(c.t, c.p, ee, T_iter, Y);
+    T_iter = temp_from_e<NS, !KCF>(c.t, c.p, ee, T_iter, Y);
   }
   __device__ __forceinline__ void done(double, double, int) const {}
 };
@@ -765,11 +766,11 @@ struct Rok4Flow {
 // in 113 ms instead of 122 ms).  The forms part only where the full form
 // breaks down: a momentum component of exactly -1e-4 makes its error term
 // (b - a) / (1e-4 a + 1e-8) 0/0 there.
-template <int NS, bool KCF>
-struct Rok4FlowSpecies : Rok4Flow<NS, KCF> {
+template <int NS, bool KCF, class CTX = DevCtx>
+struct Rok4FlowSpecies : Rok4Flow<NS, KCF, CTX> {
   const double *mom;
   __device__ __forceinline__ void rhs(const double *y, double T_iter, double *out) const {
-    krylov_rhs<NS, KCF, true>(this->c, y, mom, T_iter, out);
+    krylov_rhs<NS, KCF, !KCF>(this->c, y, mom, T_iter, out);
   }
 };
 
@@ -831,15 +832,15 @@ struct Rok4ConstP {
 };
 
 // One ROK4 flow cell; fls: the cell's fl_sav components at stride fstride (simpler == 1).
-template <int NS, bool KCF = false>
-__device__ __forceinline__ void rok4_cell(const DevCtx &c, double *VEC, double T_iter, const double *fls,
+template <int NS, bool KCF = false, class CTX>
+__device__ __forceinline__ void rok4_cell(const CTX &c, double *VEC, double T_iter, const double *fls,
                                           long long fstride, double dttry, double time_start, double time_end,
                                           int simpler) {
   if (simpler != 1) {
-    Rok4FlowSpecies<NS, KCF> f{{c}, VEC + NS};
+    Rok4FlowSpecies<NS, KCF, CTX> f{{c}, VEC + NS};
     rok4_core<NS>(c, f, VEC, T_iter, nullptr, 0, dttry, time_start, time_end, 0, c.p.ros_maxsteps);
   } else {
-    Rok4Flow<NS, KCF> f{c};
+    Rok4Flow<NS, KCF, CTX> f{c};
     rok4_core<NS + 4>(c, f, VEC, T_iter, fls, fstride, dttry, time_start, time_end, simpler, c.p.ros_maxsteps);
   }
 }

@@ -150,7 +150,9 @@ __device__ __forceinline__ double ipow(double x, int n) {
 __device__ __forceinline__ double dmax_(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ double dmin_(double a, double b) { return a < b ? a : b; }
 
-__device__ __forceinline__ void set_status(const DevPar &p, unsigned bits) {
+// PAR (here and below): DevPar, or a caller's own parameters with the same names
+template <class PAR>
+__device__ __forceinline__ void set_status(const PAR &p, unsigned bits) {
   if (p.status) atomicOr(p.status, bits);
 }
 
@@ -231,8 +233,8 @@ __device__ __forceinline__ double mix_cp2(const DevTab &t, double tt, const doub
   return cploc;
 }
 
-template <int NS>
-__device__ __forceinline__ double temp_from_poly2(const DevTab &t, const double *coef, const DevPar &p, double ee,
+template <int NS, class PAR>
+__device__ __forceinline__ double temp_from_poly2(const DevTab &t, const double *coef, const PAR &p, double ee,
                                                   double T_start, const double *Y) {
   unsigned long long hi = mid_mask<NS>(t, T_start);
   double a[6];
@@ -305,18 +307,20 @@ __device__ double mix_cp(const DevTab &t, double tt, const double *Y) {
 // get_mixture_temperature_from_e_dev (kernels_gpu.F90:6532-6622) with coef = the
 // cv table; with the cp table it is get_mixture_temperature_from_h_roe_dev
 // (:6810-6900), T from the mixture enthalpy.
-template <int NS>
-__device__ double temp_from_poly(const DevTab &t, const double *coef, const DevPar &p, double ee, double T_start,
+// P2 = false leaves the two-range form out, for a caller whose tables never have
+// it (its code and frame stay those of the general form).
+template <int NS, bool P2 = true, class PAR>
+__device__ double temp_from_poly(const DevTab &t, const double *coef, const PAR &p, double ee, double T_start,
                                  const double *Y);
-template <int NS>
-__device__ __forceinline__ double temp_from_e(const DevTab &t, const DevPar &p, double ee, double T_start,
+template <int NS, bool P2 = true, class PAR>
+__device__ __forceinline__ double temp_from_e(const DevTab &t, const PAR &p, double ee, double T_start,
                                               const double *Y) {
-  return temp_from_poly<NS>(t, t.cv, p, ee, T_start, Y);
+  return temp_from_poly<NS, P2>(t, t.cv, p, ee, T_start, Y);
 }
-template <int NS>
-__device__ double temp_from_poly(const DevTab &t, const double *coef, const DevPar &p, double ee, double T_start,
+template <int NS, bool P2, class PAR>
+__device__ double temp_from_poly(const DevTab &t, const double *coef, const PAR &p, double ee, double T_start,
                                  const double *Y) {
-  if (t.poly2) return temp_from_poly2<NS>(t, coef == t.cp ? t.cp6 : t.cv6, p, ee, T_start, Y);
+  if (P2 && t.poly2) return temp_from_poly2<NS>(t, coef == t.cp ? t.cp6 : t.cv6, p, ee, T_start, Y);
   int nrange[NS];
 #pragma unroll
   for (int k = 0; k < NS; k++) nrange[k] = 1;

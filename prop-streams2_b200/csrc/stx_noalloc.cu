@@ -22,11 +22,26 @@ static __device__ __align__(256) unsigned int g_noalloc_counter[1];
 // the end, so the 32-bit counter must stay below 2^32 with that overshoot.
 #define STX_NOALLOC_MAX_CELLS (1LL << 31)
 
+// What the chemistry reads of a context.  The out-of-line right-hand side takes it
+// by reference, so every thread keeps a local copy in the frame that callers size
+// cudaLimitStackSize by: hence not the whole DevCtx.  (Read in place through a
+// __grid_constant__ parameter it would need no copy, but the 2000 cells of an
+// H2/air flame then take 5.04 ms against 4.66.)
+struct NoallocPar {
+  double tol;
+  unsigned int *status;
+  int ros_maxsteps;
+};
+struct NoallocCtx {
+  DevTab t;
+  NoallocPar p;
+};
+
 template <int NS>
-__global__ void __launch_bounds__(128) k_rok4_noalloc(DevCtx c, double *__restrict__ w, const double *__restrict__ wa,
+__global__ void __launch_bounds__(128) k_rok4_noalloc(NoallocCtx c, DevGrid g, double *__restrict__ w,
+                                                      const double *__restrict__ wa,
                                                       const double *__restrict__ fl_sav, double dttry, double t0,
                                                       double t1, int simpler, unsigned int *counter) {
-  const DevGrid &g = c.g;
   const int NV = NS + 4;
   const double eps_Z = 5e-4;
   for (;;) {
@@ -91,18 +106,18 @@ int local_memory_ok() {
 }
 
 template <int NS>
-int launch(const DevCtx &c, cudaStream_t s, int dev, double *w, const double *wa, const double *fl_sav, double dttry,
-           double t0, double t1, int simpler, unsigned int *counter) {
+int launch(const NoallocCtx &c, const DevGrid &g, cudaStream_t s, int dev, double *w, const double *wa,
+           const double *fl_sav, double dttry, double t0, double t1, int simpler, unsigned int *counter) {
   int rc = local_memory_ok<NS>();
   if (rc != STX_OK) return rc;
   int nsm = 148, per = 1;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)k_rok4_noalloc<NS>, 128, 0);
   long long nb = (long long)nsm * (per < 1 ? 1 : per);
-  long long need = (c.g.npi + 127) / 128;
+  long long need = (g.npi + 127) / 128;
   if (nb > need) nb = need;
   if (cudaMemsetAsync(counter, 0, sizeof(unsigned int), s) != cudaSuccess) return STX_E_CUDA;
-  k_rok4_noalloc<NS><<<(int)nb, 128, 0, s>>>(c, w, wa, fl_sav, dttry, t0, t1, simpler, counter);
+  k_rok4_noalloc<NS><<<(int)nb, 128, 0, s>>>(c, g, w, wa, fl_sav, dttry, t0, t1, simpler, counter);
   return cudaGetLastError() == cudaSuccess ? STX_OK : STX_E_CUDA;
 }
 
@@ -120,11 +135,9 @@ extern "C" int stx_rosenbrock_krylov_noalloc(const stx_params *par, const stx_ta
     return STX_E_INVALID;
   const long long ncell = (long long)grid->nx * grid->ny * grid->nz;
   if (ncell > STX_NOALLOC_MAX_CELLS) return STX_E_TOO_LARGE;
-  DevCtx c;
+  NoallocCtx c{};
+  DevGrid g{};
   DevTab &t = c.t;
-  DevGrid &g = c.g;
-  DevPar &p = c.p;
-  t = DevTab{};
   t.ns = tab->ns; t.nr = tab->nr; t.icl = tab->indx_cp_l; t.icr = tab->indx_cp_r; t.nset = tab->nsetcv;
   t.ntab = tab->num_t_tab; t.ncp = t.icr - t.icl + 3; t.tmin = tab->t_min_tab; t.dtab = tab->dt_tab; t.Ru = tab->R_univ;
   t.mw = tab->mw; t.mwinv = tab->mwinv; t.rgas = tab->rgas; t.trange = tab->trange;
@@ -134,16 +147,13 @@ extern "C" int stx_rosenbrock_krylov_noalloc(const stx_params *par, const stx_ta
   t.tb_eff = tab->tb_eff; t.r_coeffs = tab->r_coeffs; t.p_coeffs = tab->p_coeffs;
   t.kc_r = tab->kc_tab;                        // reference layout, read with KCF = true
   t.n_eoi = 1;
-  g = DevGrid{};
   g.nx = grid->nx; g.ny = grid->ny; g.nz = grid->nz; g.ng = grid->ng;
   g.nxg = g.nx + 2 * g.ng; g.nyg = g.ny + 2 * g.ng; g.nzg = g.nz + 2 * g.ng;
   g.npg = (long long)g.nxg * g.nyg * g.nzg;
   g.npi = ncell;
-  p = DevPar{};
-  p.tol = par->tol_iter_nr;
-  p.ros_maxsteps = par->ros_maxsteps;
-  p.ros_eps = par->ros_eps;
-  p.status = status;
+  c.p.tol = par->tol_iter_nr;
+  c.p.status = status;
+  c.p.ros_maxsteps = par->ros_maxsteps;
   cudaStream_t s = (cudaStream_t)stream;
   // the scratch and the launch belong to the current device; a stream of
   // another device would pair it with the wrong device's counter
@@ -156,7 +166,7 @@ extern "C" int stx_rosenbrock_krylov_noalloc(const stx_params *par, const stx_ta
   int rc = counter_address(dev, &counter);
   if (rc != STX_OK) return rc;
   switch (t.ns) {
-#define X(N) case N: return launch<N>(c, s, dev, w, w_aux, fl_sav, dttry, time_start, time_end, simpler, counter);
+#define X(N) case N: return launch<N>(c, g, s, dev, w, w_aux, fl_sav, dttry, time_start, time_end, simpler, counter);
     STX_FOR_NS(X)
 #undef X
     default: return STX_E_UNSUPPORTED;
