@@ -137,8 +137,13 @@ int upload(stx_ctx *c, const T *host, size_t n, const T **out) {
 
 // The packed reaction records of chem_source_rec.  A mechanism has them when every
 // reaction is plain, three-body, Lindemann or Troe, has integer stoichiometry of
-// at most REC_SLOTS molecules a side and at most REC_NET net species; otherwise
-// t.rec stays null and the sparse lists serve it.
+// at most REC_SLOTS molecules a side, at most two of them alike, and at most REC_NET
+// net species; otherwise t.rec stays null and the sparse lists serve it.
+//
+// The records then give the bits of the lists.  A side's product is theirs because
+// a molecule that counts twice takes the first two slots: (b b) a is a (b b), which
+// the lists form, while a b b is not.  Three alike are a power there, and would make
+// net coefficients of 3, with which (nu W) q and (nu q) W round differently.
 int upload_records(stx_ctx *c, const stx_tables *tab, DevTab &t) {
   const int ns = t.ns, nr = t.nr;
   t.rec = t.rec_eff = nullptr;
@@ -169,9 +174,15 @@ int upload_records(stx_ctx *c, const stx_tables *tab, DevTab &t) {
       const double rr = tab->r_coeffs[(size_t)k * nr + r], pp = tab->p_coeffs[(size_t)k * nr + r];
       if (!(rr >= 0.0 && rr <= REC_SLOTS && pp >= 0.0 && pp <= REC_SLOTS) || rr != (int)rr || pp != (int)pp)
         return STX_OK;
-      if (nR + (int)rr > REC_SLOTS || nP + (int)pp > REC_SLOTS) return STX_OK;
-      for (int q = 0; q < (int)rr; q++) ix[nR++] = (unsigned char)k;
-      for (int q = 0; q < (int)pp; q++) ix[REC_SLOTS + nP++] = (unsigned char)k;
+      if (rr > 2.0 || pp > 2.0 || nR + (int)rr > REC_SLOTS || nP + (int)pp > REC_SLOTS) return STX_OK;
+      const auto put = [k](unsigned char *side, int &n, int count) {
+        if (count == 2 && n == 1) side[2] = side[0];    // a single one before it moves behind
+        const int at = count == 2 ? 0 : n;
+        for (int q = 0; q < count; q++) side[at + q] = (unsigned char)k;
+        n += count;
+      };
+      put(ix, nR, (int)rr);
+      put(ix + REC_SLOTS, nP, (int)pp);
       if (rr != pp) {
         if (nU == REC_NET) return STX_OK;
         ix[2 * REC_SLOTS + nU] = (unsigned char)k;

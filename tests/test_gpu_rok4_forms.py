@@ -97,3 +97,65 @@ def test_records_equal_sparse_lists(n, simpler):
             H.assert_close(got[m], ref[m], 1e-8, f"w[{m}]", floor=np.abs(ref[m]).max())
     s.close()
     o.close()
+
+
+def _with_reaction(case, reac, prod, A, kc=None, b=0.0, ER=0.0):
+    """The case with one more reaction, reac and prod: {species: molecules}; kc: its equilibrium constant
+    (None: irreversible); ER: E/R in K."""
+    tb = case.tb
+    row = lambda a, v: np.concatenate([a, np.full((1,) + a.shape[1:], v, a.dtype)])
+    rc, pc = row(tb.r_coeffs, 0), row(tb.p_coeffs, 0)
+    for c, side in ((rc, reac), (pc, prod)):
+        for k, n in side.items():
+            c[-1, tb.names.index(k)] = n
+    aa, ab, ae = row(tb.arr_a, 0), row(tb.arr_b, 0), row(tb.arr_ea, 0)
+    aa[-1, 0], ab[-1, 0], ae[-1, 0] = A, b, ER * CS.M.R_UNIV
+    tb = dataclasses.replace(tb, nr=tb.nr + 1, reac_ty=row(tb.reac_ty, 0), is_rev=row(tb.is_rev, int(kc is not None)),
+                             arr_a=aa, arr_b=ab, arr_ea=ae, falloff=row(tb.falloff, 0), tb_eff=row(tb.tb_eff, 0),
+                             r_coeffs=rc, p_coeffs=pc,
+                             kc_tab=np.concatenate([tb.kc_tab, np.full_like(tb.kc_tab[:, :1], kc or 1.0)], axis=1))
+    return _like(case, tb)
+
+
+def _like(case, tb):
+    out = CS.Case(case.cfg, tb)
+    out.w[:], out.w_aux[:] = case.w, case.w_aux
+    return out
+
+
+# sides of two and three molecules: a species that counts twice before and after a
+# single one, three different ones, and three alike (which no record holds), with
+# rates that compare with the mechanism's own
+SIDES = [({"H2": 2, "O2": 1}, {"H2O": 2}, 1e10, None), ({"O": 2, "H2": 1}, {"OH": 2}, 1e16, None),
+         ({"OH": 2}, {"O": 2, "H2": 1}, 1e13, 1e-3), ({"H": 1, "O2": 1, "N2": 1}, {"HO2": 1, "N2": 1}, 1e11, None),
+         ({"OH": 3}, {"H2O": 1, "HO2": 1}, 1e19, None), ({"H2O": 1, "HO2": 1}, {"OH": 3}, 1e13, 1e-6)]
+
+
+@pytest.mark.parametrize("n", [(8, 6, 5), (32, 20, 16)])
+@pytest.mark.parametrize("reac,prod,A,kc", SIDES)
+def test_every_form_of_a_side_has_the_bits_of_the_lists(reac, prod, A, kc, n):
+    """The simpler splitting (no shared exponential), warp and thread per cell."""
+    base = H.synthetic_case(n=n, seed=35, T0=1300.0, amp_T=400.0)
+    case = _with_reaction(base, reac, prod, A, kc)
+    lists = _like(case, _padded(case).tb)
+    (z, fz), (s, fs), (o, fo) = _source(base, 1), _source(case, 1), _source(lists, 1)
+    plain, got, ref = _rok4(z, fz, 1), _rok4(s, fs, 1), _rok4(o, fo, 1)
+    assert not np.array_equal(plain, got)            # the reaction counts
+    assert np.array_equal(got, ref)
+    for x in (z, s, o):
+        x.close()
+
+
+@pytest.mark.parametrize("reac,prod,A,kc", SIDES)
+@pytest.mark.parametrize("simpler", [0, 1])
+def test_every_form_of_a_side_in_the_warp_and_the_thread_kernel(reac, prod, A, kc, simpler):
+    case = _with_reaction(H.synthetic_case(n=(8, 6, 5), seed=35, T0=1300.0, amp_T=400.0), reac, prod, A, kc)
+    s, fs = _source(case, simpler)
+    w0 = s.w.clone()
+    out = []
+    for ctas in (0, 1):
+        s.set_tuning({"sweep_kind": [0, 0, 0], "weno_list": [1, 1, 1], "chem_ctas_per_sm": ctas})
+        s.w.copy_(w0)
+        out.append(_rok4(s, fs, simpler).copy())
+    assert np.array_equal(out[0], out[1])
+    s.close()
