@@ -144,17 +144,28 @@ int upload(stx_ctx *c, const T *host, size_t n, const T **out) {
 // a molecule that counts twice takes the first two slots: (b b) a is a (b b), which
 // the lists form, while a b b is not.  Three alike are a power there, and would make
 // net coefficients of 3, with which (nu W) q and (nu q) W round differently.
+//
+// rec_tmin keeps |b ln T - E / (R T)| of every rate below 700 from there to 1e6 K:
+// arrhenius_dd takes the exponential of the whole, which beyond 709 overflows (or
+// goes subnormal) where the power and the exponential, each with A, need not.
 int upload_records(stx_ctx *c, const stx_tables *tab, DevTab &t) {
   const int ns = t.ns, nr = t.nr;
-  t.rec = t.rec_eff = nullptr;
-  t.rec_es = (ns + 1) & ~1;
+  t.rec = nullptr;
+  t.rec_tmin = 1.0;
   if (ns > 200) return STX_OK;
-  std::vector<double> rec((size_t)nr * REC_N, 0.0), eff((size_t)nr * t.rec_es, 0.0);
+  std::vector<double> rec((size_t)nr * (REC_N + rec_es(ns)), 0.0);
+  double *eff = &rec[(size_t)nr * REC_N];
   for (int r = 0; r < nr; r++) {
     double *R = &rec[(size_t)r * REC_N];
     const int ty = tab->reac_ty[r];
     if (ty < 0 || ty > 3) return STX_OK;
     int cls = ty == 0 ? REC_PLAIN : ty == 1 ? REC_TB : ty == 2 ? REC_LIND : REC_TROE;
+    for (int q = r; q <= (ty < 2 ? r : nr + r); q += nr) {
+      const double room = 700.0 - std::fabs(tab->arr_b[q]) * std::log(1e6);
+      const double tmin = std::fabs(tab->arr_ea[q]) / tab->R_univ / room;
+      if (!(room > 0.0 && tmin < 1e6)) return STX_OK;
+      if (tmin > t.rec_tmin) t.rec_tmin = tmin;
+    }
     R[0] = tab->arr_a[r]; R[1] = tab->arr_b[r]; R[2] = -tab->arr_ea[r];
     R[4] = tab->arr_a[nr + r]; R[5] = tab->arr_b[nr + r]; R[6] = -tab->arr_ea[nr + r];
     if (ty == 3) {
@@ -188,14 +199,13 @@ int upload_records(stx_ctx *c, const stx_tables *tab, DevTab &t) {
         ix[2 * REC_SLOTS + nU] = (unsigned char)k;
         R[8 + nU++] = (pp - rr) * tab->mw[k];
       }
-      eff[(size_t)r * t.rec_es + k] = tab->tb_eff[(size_t)k * nr + r];
+      eff[(size_t)r * rec_es(ns) + k] = tab->tb_eff[(size_t)k * nr + r];
     }
     const int flag[2] = {cls | (tab->is_rev[r] == 1) << 8 | nU << 16, 0};   // low word first
     std::memcpy(R + 7, flag, sizeof flag);
     std::memcpy(R + 14, ix, sizeof ix);
   }
-  int rc = upload(c, rec.data(), rec.size(), &t.rec);
-  return rc ? rc : upload(c, eff.data(), eff.size(), &t.rec_eff);
+  return upload(c, rec.data(), rec.size(), &t.rec);
 }
 
 bool ns_supported(int ns) {

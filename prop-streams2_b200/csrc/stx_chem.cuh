@@ -85,9 +85,6 @@ __device__ __forceinline__ double arrhenius_dd(double A, double b, double nE, do
   return A * fma(x, e, x);
 }
 
-// the temperatures the packed records serve (NaN: no)
-__device__ __forceinline__ bool rate_range(double tt) { return tt >= 1.0 && tt <= 1.0e6; }
-
 // Rate constants of reaction lr at T (kernels_gpu.F90:9266-9330): kf from the
 // Arrhenius, Lindemann, Troe or SRI form (tbs is the third-body concentration
 // sum the fall-off forms use), kb = kf / K_c with K_c interpolated in the 1-K
@@ -301,9 +298,12 @@ __device__ __forceinline__ double rec_kf(const DevTab &t, int lr, int cls, doubl
   return kinf * (rpres / (1.0 + rpres)) * (DD ? exp10(ex) : pow(10.0, ex));
 }
 
-// whether the records serve temperature tt: a constant Fcent is its limit over
-// rate_range only (anything else takes the general tables)
-__device__ __forceinline__ bool rec_range(const DevTab &t, double tt) { return t.rec != nullptr && rate_range(tt); }
+// Whether the records serve temperature tt (NaN: no; anything else takes the sparse
+// lists).  A constant Fcent is its limit up to 1e6 K only, and below rec_tmin the
+// exponential of arrhenius_dd could leave the range of a double.
+__device__ __forceinline__ bool rec_range(const DevTab &t, double tt) {
+  return t.rec != nullptr && tt >= t.rec_tmin && tt <= 1.0e6;
+}
 
 // The terms of chem_source_sp over the records.  conc and rhs are per-thread
 // rows with stride S and NS + 1 entries: conc[NS] holds 1, rhs[NS] is scratch.
@@ -311,7 +311,8 @@ __device__ __forceinline__ bool rec_range(const DevTab &t, double tt) { return t
 // loaded one reaction ahead.
 template <int NS, int S, bool DD>
 __device__ __forceinline__ void chem_source_rec(const DevTab &t, double tt, const double *conc, double *rhs) {
-  const int nr = t.nr, es = t.rec_es;
+  const int nr = t.nr;
+  constexpr int es = rec_es(NS);
   const double rt = 1.0 / (t.Ru * tt);
   double lh = 0.0, ll = 0.0;
   if (DD) log_dd(tt, lh, ll);
@@ -333,7 +334,7 @@ __device__ __forceinline__ void chem_source_rec(const DevTab &t, double tt, cons
     double tbs = 1.0;
     if (cls != REC_PLAIN) {
       tbs = 0.0;
-      const double *ef = t.rec_eff + (long long)lr * es;
+      const double *ef = t.rec + (nr * REC_N + lr * es);
 #pragma unroll
       for (int k = 0; k < NS; k++) tbs = tbs + ldg(ef + k) * conc[k * S];
     }

@@ -34,6 +34,7 @@ __host__ __device__ constexpr int xsweep_block(int ns) { return ns > 20 ? 64 : 1
 #define REC_N 16
 #define REC_SLOTS 3        // reactant (or product) molecules of a reaction
 #define REC_NET 6          // net species of a reaction
+__host__ __device__ constexpr int rec_es(int ns) { return (ns + 1) & ~1; }   // stride of a third-body row
 enum { REC_PLAIN = 0, REC_TB = 1, REC_LIND = 2, REC_TROE_C = 3, REC_TROE = 4 };
 
 struct DevTab {
@@ -69,10 +70,11 @@ struct DevTab {
   int poly2;
   double umid;
   const double *cp6, *cv6, *cpi6; // (6, ns, nset): the powers 0..4 and the constant of cp, cv and cpi
-  // packed reaction records [lr][REC_N] and third-body rows [lr][rec_es] of
-  // chem_source_rec; null where a reaction does not fit the record
-  const double *rec, *rec_eff;
-  int rec_es;
+  // packed reaction records [lr][REC_N] and, behind them, third-body rows
+  // [lr][rec_es(ns)] of chem_source_rec; null where a reaction does not fit the
+  // record.  They serve temperatures from rec_tmin.
+  const double *rec;
+  double rec_tmin;
   int n_eoi;
   const double *aw_eoi, *coeff_eoi, *beta0;
   const int *nainsp;

@@ -202,7 +202,7 @@ __device__ __forceinline__ double production_w(const DevTab &t, double tt, doubl
       double tbs = 1.0;
       if (cls != REC_PLAIN) {
         tbs = 0.0;
-        const double *ef = t.rec_eff + (long long)lr * t.rec_es;
+        const double *ef = t.rec + (nr * REC_N + lr * rec_es(NS));
 #pragma unroll
         for (int k = 0; k < NS; k++) tbs = tbs + ldg(ef + k) * conc[k];
       }

@@ -159,3 +159,20 @@ def test_every_form_of_a_side_in_the_warp_and_the_thread_kernel(reac, prod, A, k
         out.append(_rok4(s, fs, simpler).copy())
     assert np.array_equal(out[0], out[1])
     s.close()
+
+
+@pytest.mark.parametrize("n", [(8, 6, 5), (32, 20, 16)])
+@pytest.mark.parametrize("simpler", [0, 1])
+def test_rates_beyond_the_records_temperatures_take_the_lists(simpler, n):
+    """A = 1e-307, b = 22, E/R = -728000 K: 5e4 at 1300 K, where b ln T - E / (R T) is
+    717 and its exponential overflows.  The records' lower limit, 1840 K here, leaves
+    such cells to the power and the exponential of the lists."""
+    base = H.synthetic_case(n=n, seed=37, T0=1300.0, amp_T=0.0)
+    case = _with_reaction(base, {"H2": 1, "O2": 1}, {"OH": 2}, 1e-307, b=22.0, ER=-728000.0)
+    lists = _like(case, _padded(case).tb)
+    (z, fz), (s, fs), (o, fo) = _source(base, simpler), _source(case, simpler), _source(lists, simpler)
+    plain, got, ref = _rok4(z, fz, simpler), _rok4(s, fs, simpler), _rok4(o, fo, simpler)
+    assert np.isfinite(ref).all() and not np.array_equal(plain, ref)
+    assert np.array_equal(got, ref)
+    for x in (z, s, o):
+        x.close()
