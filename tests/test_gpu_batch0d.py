@@ -95,20 +95,15 @@ def test_batch_reactor_conserves_enthalpy_and_mass(batch):
 
 def test_warp_and_thread_reactor_kernels_agree(batch, monkeypatch):
     """The warp-per-reactor kernel (default where the mechanism fits) and the
-    thread-per-reactor kernel integrate the same reactors to the same answer
-    within the adaptive integration's conditioning: their Krylov dot products
-    are summed in different orders, and a last-bit change moves an ignition
-    time by up to ~5e-4 relative (the module's note), so two such changes are
-    allowed 2e-3 at most and 1e-5 in the median."""
+    thread-per-reactor kernel integrate the same reactors with the same
+    operations in the same order: the same bits."""
     T0, p0, Y0 = sample_h2air(48, 31, batch.mech, T_range=(1100.0, 1500.0))
     w = {k: v.cpu().numpy() for k, v in batch.integrate(T0, p0, Y0, T_MAX, DTTRY, 1.05, 2.0, MAXSTEPS).items()}
     monkeypatch.setenv("STX_BATCH0D_KERNEL", "thread")
     t = {k: v.cpu().numpy() for k, v in batch.integrate(T0, p0, Y0, T_MAX, DTTRY, 1.05, 2.0, MAXSTEPS).items()}
-    ign = t["t_ign"] > 0
-    assert np.array_equal(w["t_ign"] > 0, ign)
-    r = np.abs(w["t_ign"][ign] - t["t_ign"][ign]) / t["t_ign"][ign]
-    assert r.max() < 2e-3 and np.median(r) < 1e-5, (r.max(), np.median(r))
-    assert np.max(np.abs(w["T"] - t["T"]) / t["T"]) < 1e-3
+    assert (w["t_ign"] > 0).sum() > 40
+    for k in ("Y", "T", "t_ign", "t_end", "nsteps"):
+        assert np.array_equal(w[k], t[k]), k
 
 
 def test_split_form_against_oracle(batch):

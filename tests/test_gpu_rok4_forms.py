@@ -21,7 +21,9 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():
     pytest.skip("no CUDA device", allow_module_level=True)
 
+from driver import OracleSolver  # noqa: E402
 from stx import case as CS  # noqa: E402
+from stx import mech as M  # noqa: E402
 from stx.native import check  # noqa: E402
 from stx.solver import Solver  # noqa: E402
 
@@ -176,3 +178,81 @@ def test_rates_beyond_the_records_temperatures_take_the_lists(simpler, n):
     assert np.array_equal(got, ref)
     for x in (z, s, o):
         x.close()
+
+
+# one cp range boundary for all species and plain, three-body and Troe reactions (9, 11);
+# several boundaries, Lindemann and a side with a repeated species (14, and 13 without He)
+MECHS = ["h2air_9sp", "flame_11sp", "keromnes_13sp", "keromnes_14sp"]
+
+
+@pytest.fixture
+def any_mech(monkeypatch):
+    full = H.mechanism
+
+    def pick(name):
+        if name != "keromnes_13sp":
+            return full(name)
+        m = full("keromnes_14sp")
+        return M.restrict_species(m, [x for x in m.names if x != "HE"])
+
+    monkeypatch.setattr(H, "mechanism", pick)
+
+
+def _tune(s, ctas):
+    s.set_tuning({"sweep_kind": [0, 0, 0], "weno_list": [1, 1, 1], "chem_ctas_per_sm": ctas})
+
+
+@pytest.mark.parametrize("mech", MECHS)
+@pytest.mark.parametrize("simpler", [0, 1])
+def test_every_mechanism_warp_thread_and_lists(any_mech, mech, simpler):
+    """431 cells (no multiple of a warp or a CTA): the warp kernel, the thread kernel's
+    persistent and plain launches and, without the shared exponential, the lists."""
+    case = H.synthetic_case(n=(431, 1, 1), mech=mech, seed=39, T0=1350.0, amp_T=1400.0)
+    s, fs = _source(case, simpler)
+    w0 = s.w.clone()
+    out = []
+    for ctas in (0, 1, -1):
+        _tune(s, ctas)
+        s.w.copy_(w0)
+        out.append(_rok4(s, fs, simpler).copy())
+    assert not np.array_equal(out[0], case.interior(w0.cpu().numpy())) and np.isfinite(out[0]).all()
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    o, fo = _source(_like(case, _padded(case).tb), simpler)
+    for ctas in (0, 1):
+        _tune(o, ctas)
+        o.w.copy_(w0)
+        ref = _rok4(o, fo, simpler)
+        if simpler:
+            assert np.array_equal(out[0], ref)
+        else:                            # the bound of test_records_equal_sparse_lists
+            for m in range(case.nv):
+                H.assert_close(out[0][m], ref[m], 1e-8, f"w[{m}]", floor=np.abs(ref[m]).max())
+    s.close()
+    o.close()
+
+
+@pytest.mark.parametrize("mech", MECHS)
+@pytest.mark.parametrize("ctas", [0, 1, -1])
+@pytest.mark.parametrize("simpler", [0, 1])
+def test_every_kernel_against_the_oracle(any_mech, mech, ctas, simpler):
+    """A short window of each kernel against the FP64 oracle, to 1e-9 of a component
+    (one or two steps: rounding enters through exp, pow and log10 alone)."""
+    case = H.synthetic_case(n=(10, 8, 6), mech=mech, seed=10, T0=1300.0, amp_T=200.0)
+    s = Solver(case)
+    o = OracleSolver(case, threads=8)
+    o.update_ghost(1)
+    o.compute_aux(1, 1)
+    o.fl_sav[:] = 1e-3 * np.random.default_rng(12).standard_normal(o.fl_sav.shape)
+    s.w.copy_(torch.from_numpy(o.w))
+    s.w_aux.copy_(torch.from_numpy(o.w_aux))
+    s.fl_sav.copy_(torch.from_numpy(o.fl_sav))
+    _tune(s, ctas)
+    p = lambda a: C.c_void_p(a.ctypes.data)
+    w0 = case.interior(o.w).copy()
+    o.lib.ox_rosenbrock_krylov(o.ctx, p(o.w), p(o.w_aux), p(o.fl_sav), DT, 0.0, DT, simpler)
+    wg, wo = _rok4(s, s.fl_sav, simpler), case.interior(o.w)
+    assert not np.array_equal(wo, w0)
+    for m in range(case.nv):
+        H.assert_close(wg[m], wo[m], 1e-9, f"w[{m}]", floor=1e-9 * np.abs(wo[:case.ns]).max() if m < case.ns else None)
+    s.close()
+    o.close()
