@@ -24,7 +24,11 @@
 // window of H2/air cells on a B200, thread against warp: 1024 cells 791 / 193 us,
 // 4096 814 / 309, 8192 811 / 548, 12288 825 / 760, 16384 825 / 986 (simpler
 // splitting 1033 / 227, 1052 / 362, 1055 / 652, 1066 / 919, 1065 / 1184).  The lines
-// cross near 13000; cells that need more steps move it, hence the margin.
+// cross near 13000 there.  Windows of more steps, whose cells differ in number, move
+// the crossing: at 8192 cells 2e-7 s 7.03 / 7.30 ms (simpler 9.04 / 8.89), 2e-6 s
+// 133 / 119; 11 species 7.77 / 7.70 and 150 / 125; 14 species and 37 reactions 63.6 /
+// 32.0 and 289 / 138 (13 species alike).  At 6144 cells and fewer the warp is ahead in
+// all of these (9 species, 2e-7 s: 6.98 / 5.63).
 #ifndef STX_ROK4_WARP_CELLS
 #define STX_ROK4_WARP_CELLS 8192
 #endif

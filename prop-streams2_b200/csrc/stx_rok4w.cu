@@ -7,9 +7,9 @@
 // some 1e5 cycles for a step of one state.  Here a warp integrates one state:
 //  * lane m holds component m of every vector (state, Krylov basis, stages);
 //    dot products and norms sum the lanes' products in component order, by
-//    shuffles that do not depend on one another and a chain of adds (no longer
-//    than a butterfly's five shuffle-and-add rounds), so every lane has the bits
-//    of the thread kernels' loops;
+//    shuffles that do not depend on one another and a chain of adds, one per
+//    component, so every lane has the bits of the thread kernels' loops (a
+//    butterfly would take five rounds, in another order);
 //  * the right-hand side evaluates the reaction rates one reaction per lane
 //    (the per-reaction arithmetic of chem_source_rec or chem_source_sp), then
 //    lane k sums its species' terms in ascending reaction order from shared
@@ -342,7 +342,10 @@ struct Rok4FlowW {
 // One warp per flow cell (k_rok4's work on a small grid).  Bound by the latency of
 // a cell's chain of right-hand sides: the budget of four CTAs per SM (128 registers, some
 // spilled outside the right-hand side) keeps 2368 cells resident at once.  4096
-// H2/air cells: 309 us against 814 us with a thread per cell.
+// H2/air cells: 309 us against 814 us with a thread per cell.  Budgets of 2, 3, 4, 5
+// and 6 CTAs, one 2e-7 s window on a B200: 1024 H2/air cells 1.50, 1.55, 1.66, 1.77,
+// 1.84 ms; 4096 4.98, 4.26, 3.95, 4.24, 4.41; 8192 8.86, 7.53, 7.36, 7.41, 7.52; 4096
+// cells of 14 species 22.6, 20.0, 19.6, 22.4, 23.7.
 template <int NS>
 __global__ void __launch_bounds__(128, 4)
     k_rok4_w(DevCtx c, const DevCtx *__restrict__ cg, double *__restrict__ w, const double *__restrict__ wa,
