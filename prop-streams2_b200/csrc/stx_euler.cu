@@ -611,10 +611,16 @@ template <int NS> struct YZTile {
 };
 #define YZ_TI (YZTile<NS>::TI)
 #define YZ_TF (YZTile<NS>::TF)
+// CTAs per SM: two are stated where the compiler, left to itself, takes 254 registers,
+// which is one: 14 species, and 13 in the z sweep.  14 species on 96 x 64 x 64 cells, y
+// and z: 1.01 and 1.05 ms against 1.29 and 1.31; on 32 x 32 x 16, which leaves the
+// second place empty, 0.127 and 0.130 against 0.109 and 0.104.  Elsewhere none are
+// (0): the 128 registers that it takes by itself are 2 to 6 % faster than two stated,
+// and one stated makes them 254 (9 species 0.93 ms against 0.69).
 template <int NS, int DIR, typename R>
-__global__ void __launch_bounds__(YZ_TI * YZ_TF) k_euler_yz(DevCtx c, const DevCtx *__restrict__ cg,
-                                                           const double *__restrict__ wa, double *__restrict__ fl,
-                                                           int nmin, int nmax, int overwrite) {
+__global__ void __launch_bounds__(YZ_TI * YZ_TF, NS == 14 || (NS == 13 && DIR == 2) ? 2 : 0)
+    k_euler_yz(DevCtx c, const DevCtx *__restrict__ cg, const double *__restrict__ wa, double *__restrict__ fl,
+               int nmin, int nmax, int overwrite) {
   const DevGrid &g = c.g;
   const int NV = NS + 4;
   __shared__ R sf[NV][YZ_TF][YZ_TI];
